@@ -38,7 +38,7 @@ UNITS = {
     "vts.cu": [],
     "slab.cu": [],
 }
-HEADERS = ["lattice.cuh", "kernels.cuh", "kernels_tma.cuh", "tma.cuh", "launch.cuh", "engine.hpp", "config.hpp",
+HEADERS = ["lattice.cuh", "kernels.cuh", "kernels_split.cuh", "kernels_tma.cuh", "tma.cuh", "launch.cuh", "engine.hpp", "config.hpp",
            "solver.hpp", "dual.cuh", "adjoint.cuh"]
 
 

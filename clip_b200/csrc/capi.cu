@@ -148,9 +148,7 @@ int clipb::solver_create(const CaseConfig& cfg, int precision, clipb_solver** ou
     }
     s->kt = precision == CLIPB_FP64 ? kernels_fp64() : (precision == CLIPB_FP32 ? kernels_fp32() : kernels_fp16());
     st.seg = 0;
-    // default launch variant: FP32/FP16 keep g of the next plane in registers (2D), FP64
-    // re-pulls it; clipb_autotune can pick another one
-    st.variant = 0;
+    st.variant = s->kt.default_variant(st);  // clipb_autotune can pick another one
 
     const int Q = c.dim == 3 ? 19 : 9;
     // the step kernels index every buffer with 32-bit element offsets
@@ -182,6 +180,7 @@ int clipb::solver_create(const CaseConfig& cfg, int precision, clipb_solver** ou
         }
     }
     if ((rc = s->alloc(&st.p, aux))) return rc;
+    if (c.dim == 3 && precision != CLIPB_FP64 && (rc = s->alloc(&st.cw, (size_t)g.ps * 8))) return rc;
     if ((rc = s->alloc((void**)&st.c0, (size_t)g.ps * sizeof(double)))) return rc;
     st.red_blocks = 8 * 148;  // monitor blocks: a fixed count keeps the sums deterministic
     if ((rc = s->alloc((void**)&st.red, (size_t)2 * st.red_blocks * sizeof(double)))) return rc;
@@ -701,7 +700,7 @@ int clipb_autotune(clipb_solver* s, int trial_steps, int* best_variant, int* bes
     for (int v = 0; v < nv; ++v) {
         if (!s->kt.available(s->st, v)) continue;
         for (int seg : segs)
-            if (seg <= n_march || seg == segs.front()) cands.emplace_back(v, seg);
+            if (seg == segs.front() || (seg <= n_march && s->kt.marches(s->st, v))) cands.emplace_back(v, seg);
     }
     std::vector<float> ms_best(cands.size(), 1e30f);
     for (int pass = 0; pass < 2; ++pass) {

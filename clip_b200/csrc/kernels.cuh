@@ -602,6 +602,7 @@ struct StepArgs {
     // the mass and kinetic energy of the step's stored c and u, as monitor_partials forms
     // them per node
     double* mon;
+    typename PR::Ring* cw;  // two-pass step: this step's c of every node and ghost node
 };
 
 // Shift of direction q as dest_shift computes it, evaluated when it is needed.
@@ -610,6 +611,20 @@ __device__ __forceinline__ V dest_shift_q(int q, unsigned dmask, V cown, Cfun Cd
     using L = Lat<DIM>;
     if constexpr (!PR::kShift) return cown;
     else return (dmask & (1u << q)) ? cown : Cd(L::ex(q), L::ey(q), DIM == 3 ? L::ez(q) : 0);
+}
+
+// Mass and kinetic energy of one node from its stored c and u, in FP64.
+template <int DIM, class PR>
+__device__ __forceinline__ void node_monitors(const StepArgs<PR>& a, typename PR::A c, const typename PR::T* u, double* mon) {
+    const double cs = double(c);
+    double u2 = 0.0;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        const double v = double(typename PR::A(u[d]));
+        u2 += v * v;
+    }
+    mon[0] = cs;
+    mon[1] = 0.5 * (a.phys.RhoL + cs * a.phys.drho) * u2;
 }
 
 // Macroscopic update and the next collision of one interior node, then its stores.
@@ -653,8 +668,7 @@ __device__ __forceinline__ void update_node(const StepArgs<PR>& a, const Codec<P
 #pragma unroll
         for (int q = 0; q < Q; ++q) cd.store_f(a.fout + (self + unsigned(q) * unsigned(g.ps)), fo[q]);
     } else {
-        T p;
-        lean_update<DIM>(PT, fpost, gpost, delta, c_old, c, mu, dc, u, cdest, p, [&](int q, T fo, TP go) {
+        lean_update<DIM>(PT, lean_moments<DIM>(fpost), gpost, delta, c_old, c, mu, dc, u, cdest, [&](int q, T fo, TP go) {
             cd.store_dev(a.gout + (self + unsigned(q) * unsigned(g.ps)), go);
             cd.store_f(a.fout + (self + unsigned(q) * unsigned(g.ps)), fo);
         });
@@ -662,17 +676,7 @@ __device__ __forceinline__ void update_node(const StepArgs<PR>& a, const Codec<P
 #pragma unroll
     for (int d = 0; d < DIM; ++d) U[self + unsigned(d) * unsigned(g.ps)] = A(u[d]);
     a.cout[self] = A(c);
-    if (mon) {
-        const double cs = double(A(c));
-        double u2 = 0.0;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-            const double v = double(A(u[d]));
-            u2 += v * v;
-        }
-        mon[0] = cs;
-        mon[1] = 0.5 * (a.phys.RhoL + cs * a.phys.drho) * u2;
-    }
+    if (mon) node_monitors<DIM, PR>(a, A(c), u, mon);
 }
 
 // Sum of the Q pulled values in ascending q (the order of ring_c and of lean_update's delta).
@@ -844,6 +848,26 @@ __device__ __forceinline__ void halo_coords(int h, int& hx, int& hy) {
     else { hx = HX - 1; hy = 1 + (h - 2 * HX - TY); }
 }
 
+// Monitored step: each warp (32 consecutive x of one row) sums its nodes' mass and kinetic
+// energy in a fixed tree into one entry per row segment, so the result does not depend on the
+// tile shape or the planes per CTA.
+template <class PR>
+__device__ __forceinline__ void store_monitor_row(const StepArgs<PR>& a, int tx, int x0, int y, int z, const double* mon) {
+    const Geom& g = a.g;
+    double m = mon[0], k = mon[1];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        m += __shfl_down_sync(0xffffffffu, m, off);
+        k += __shfl_down_sync(0xffffffffu, k, off);
+    }
+    const int nxs = (g.n[0] + 31) / 32, xs = (x0 - 1 + (tx & ~31)) / 32;
+    if ((tx & 31) == 0 && y <= g.n[1] && xs < nxs) {
+        const long long row = ((long long)(z - g.zlo) * g.n[1] + (y - 1)) * nxs + xs;
+        a.mon[2 * row] = m;
+        a.mon[2 * row + 1] = k;
+    }
+}
+
 // The 3D step of one CTA with loads straight from global memory.  `ring` is the CTA's
 // 4-plane phase-field ring of (TX+2)*(TY+2) values.  Only nodes next to a boundary take the
 // boundary-aware pull.  Every per-node code path appears once (one box loop, one update),
@@ -957,23 +981,7 @@ __device__ __forceinline__ void step3d_body(const StepArgs<PR>& a, int seg, int 
             }
             if (kOpen && g.fc[0]) store_open_u<3, PR>(g, a.par, x, y, z, a.u, self);
         }
-        // monitored step: each warp (32 consecutive x of one row) sums its nodes' mass and
-        // kinetic energy in a fixed tree into one entry per row segment, so the result does
-        // not depend on the tile shape or the planes per CTA
-        if (kMon && z >= z0) {
-            double m = mon2[0], k = mon2[1];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                m += __shfl_down_sync(0xffffffffu, m, off);
-                k += __shfl_down_sync(0xffffffffu, k, off);
-            }
-            const int nxs = (g.n[0] + 31) / 32, xs = (x0 - 1 + (tx & ~31)) / 32;
-            if ((tx & 31) == 0 && y <= g.n[1] && xs < nxs) {
-                const long long row = ((long long)(z - g.zlo) * g.n[1] + (y - 1)) * nxs + xs;
-                a.mon[2 * row] = m;
-                a.mon[2 * row + 1] = k;
-            }
-        }
+        if (kMon && z >= z0) store_monitor_row(a, tx, x0, y, z, mon2);
         if constexpr (kKeepG) {
 #pragma unroll
             for (int q = 0; q < Q; ++q) gcur[q] = gnext[q];

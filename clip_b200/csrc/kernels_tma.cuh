@@ -23,7 +23,7 @@
 // itself before the block drains.
 #pragma once
 
-#include "kernels.cuh"
+#include "kernels_split.cuh"
 #include "tma.cuh"
 
 namespace clipb {

@@ -496,7 +496,7 @@ __device__ __forceinline__ void unit_normal(const float* dc, float* n) {
 // literal transforms (macroscopic / collide_f) for bit-exact parity.
 // The update is arranged per pair (q, opposite q): the pair's sum and difference give the
 // moments, and each output splits into a part even in e_q and a part odd in e_q.
-//   f       : streamed f (p, j and Pi moments)
+//   m       : moments of the streamed f
 //   d(q)    : streamed g minus w_q c_old (c_old: this node's stored c of the previous step)
 //   delta   : sum d in the order d_0 + d_1 + ... (the phase-field sum of the node's c)
 //   c       : this step's c (= c_old + delta, rounded as stored);  mu, dc: its stencils
@@ -522,14 +522,17 @@ __device__ __forceinline__ void unit_normal(const float* dc, float* n) {
 // multiply-add is written out (fmaf) and the FP32 units are compiled without contraction, so
 // each launch shape rounds the same way; the three quotients are the units' fast division
 // (-prec-div=false), one fixed instruction sequence wherever the update is inlined.
-template <int DIM, class Dq, class Cq, class Out>
-__device__ __forceinline__ void lean_update(const Phys<float>& P, const float* f, Dq d, float delta, float c_old,
-                                            float c, float mu, const float* dc, float* u, Cq cdest, float& p_out,
-                                            Out out) {
+//
+// Moments of the streamed f that the update needs (the f themselves are not used further).
+struct Moments {
+    float p, j[3], Pi[6];  // Pi: xx yy zz xy xz yz
+};
+template <int DIM>
+__device__ __forceinline__ Moments lean_moments(const float* f) {
     using L = Lat<DIM>;
     constexpr int Q = L::Q;
     float p = f[0], j[3] = {0.f, 0.f, 0.f};
-    float Pi[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // xx yy zz xy xz yz
+    float Pi[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int q = 1; q < Q; ++q) {
         const int o = opposite<DIM>(q);
@@ -547,6 +550,16 @@ __device__ __forceinline__ void lean_update(const Phys<float>& P, const float* f
         if (DIM == 3 && ex * ez) Pi[4] += ex * ez > 0 ? s : -s;
         if (DIM == 3 && ey * ez) Pi[5] += ey * ez > 0 ? s : -s;
     }
+    return Moments{p, {j[0], j[1], j[2]}, {Pi[0], Pi[1], Pi[2], Pi[3], Pi[4], Pi[5]}};
+}
+
+template <int DIM, class Dq, class Cq, class Out>
+__device__ __forceinline__ void lean_update(const Phys<float>& P, const Moments& m, Dq d, float delta, float c_old, float c,
+                                            float mu, const float* dc, float* u, Cq cdest, Out out) {
+    using L = Lat<DIM>;
+    constexpr int Q = L::Q;
+    const float p = m.p;
+    const float *j = m.j, *Pi = m.Pi;
     const float rho = fmaf(c, P.drho, P.RhoL);
     // relaxation time, clamped outside [0, 1] (NsAllen.cu:418-425)
     const float tau = c < 0.f ? P.tauL : (c > 1.f ? P.tauH : fmaf(c, P.dtau, P.tauL));
@@ -658,7 +671,6 @@ __device__ __forceinline__ void lean_update(const Phys<float>& P, const float* f
         out(q, fmaf(w3, eU, fmaf(w, pe, fF)), fmaf(omw, d(q), fmaf(w, ge + (c_old - cdest(q)), ga)));
         out(o, fmaf(-w3, eU, fmaf(w, pe, -fF)), fmaf(omw, d(o), fmaf(w, ge + (c_old - cdest(o)), -ga)));
     }
-    p_out = p;
 }
 
 // Error-free sum: hi + lo == a + b exactly (Knuth's TwoSum, round-to-nearest).

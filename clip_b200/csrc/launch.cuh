@@ -8,6 +8,7 @@
 #include <cstring>
 
 #include "kernels.cuh"
+#include "kernels_split.cuh"
 #include "kernels_tma.cuh"
 
 namespace clipb {
@@ -57,6 +58,7 @@ struct Launch {
         a.pop_scale = st.pop_scale;
         a.par = in;
         a.mon = st.mon_rows;
+        a.cw = static_cast<typename PR::Ring*>(st.cw);
         return a;
     }
 
@@ -142,11 +144,8 @@ struct Launch {
                 if (ek == cudaSuccess)
                     ek = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
             };
-            allow(step3d_smemkeep_kernel<PR, 32, 8, 2, false>, smemkeep_bytes<8>());
             allow(step3d_smemkeep_kernel<PR, 32, 8, 3, false>, smemkeep_bytes<8>());
-            allow(step3d_smemkeep_kernel<PR, 32, 8, 2, true>, smemkeep_bytes<8>());
             allow(step3d_smemkeep_kernel<PR, 32, 8, 3, true>, smemkeep_bytes<8>());
-            allow(step3d_smemkeep_kernel<PR, 32, 8, 2, false, true>, smemkeep_bytes<8>());
             allow(step3d_smemkeep_kernel<PR, 32, 8, 3, false, true>, smemkeep_bytes<8>());
             if (ek != cudaSuccess) return ek;
             auto* h = new StageHost();
@@ -259,6 +258,33 @@ struct Launch {
         }
     }
 
+    // The two-pass step (kernels_split.cuh).
+    template <int DIM, bool kOpen>
+    static void go_split(const DevState& st, const StepArgs<PR>& a, cudaStream_t s) {
+        const Geom& g = st.g;
+        const int nx = (g.n[0] + 31) / 32;
+        const int z0 = DIM == 3 ? g.zlo - 1 : 0, nz = DIM == 3 ? g.zhi - g.zlo + 1 : 1;
+        if constexpr (DIM == 3 && !kOpen && !PR::kExact) {
+            using L = Lat<3>;
+            PullPtrs<PR> ptr;
+            for (int q = 0; q < L::Q; ++q) {
+                const long long from = q * g.ps - L::ex(q) - L::ey(q) * g.sy - L::ez(q) * g.sz;
+                ptr.f[q] = a.fin + from;
+                ptr.g[q] = a.gin + from;
+                ptr.fo[q] = a.fout + q * g.ps;
+                ptr.go[q] = a.gout + q * g.ps;
+            }
+            constexpr int TY = 4;
+            const dim3 gu(nx, (g.n[1] + TY - 1) / TY, nz), bu(32, TY);
+            (void)launch_chained(phase3_kernel<PR>, dim3(nx, (g.n[1] + 2 + 7) / 8, nz + 2), dim3(32, 8), 0, s, a, ptr, z0);
+            if (a.mon) (void)launch_chained(update3_kernel<PR, TY, true>, gu, bu, 0, s, a, ptr, z0 + 1);
+            else (void)launch_chained(update3_kernel<PR, TY, false>, gu, bu, 0, s, a, ptr, z0 + 1);
+        } else {
+            phase_kernel<DIM, PR, kOpen><<<dim3(nx, (g.n[1] + 2 + 7) / 8, DIM == 3 ? nz + 2 : 1), dim3(32, 8), 0, s>>>(a, z0);
+            update_kernel<DIM, PR, kOpen><<<dim3(nx, (g.n[1] + 3) / 4, nz), dim3(32, 4), 0, s>>>(a);
+        }
+    }
+
     template <int TX, bool kKeep, bool kOpen>
     static void go2(const DevState& st, const StepArgs<PR>& a, cudaStream_t s) {
         const Geom& g = st.g;
@@ -271,8 +297,8 @@ struct Launch {
     // autotuner in capi.cu picks one per solver.  kKeepG2/kKeepG3 = false restricts a
     // precision to the re-pulling variants (FP64: registers).
     // Variants 5 and 6 (FP32/FP16) are the staged step with 32 x 8 and 32 x 4 tiles.
-    // Variants 7 and 8 (FP32/FP16) keep the next plane's g in shared memory, with at least
-    // 2 and 3 resident 32 x 8 blocks per SM.
+    // Variant 7 (FP32/FP16) is the two-pass step, variant 8 keeps the next plane's g in shared
+    // memory, with at least 3 resident 32 x 8 blocks per SM.
     // Variant 9 (FP32/FP16) is the staged step with g by bulk copies and f pulled from global
     // memory, at least 2 resident 32 x 8 blocks per SM.
     static constexpr int kVariants3 = kStaged ? 10 : 5, kVariants2 = 4;
@@ -292,7 +318,9 @@ struct Launch {
                 case 6:
                     if constexpr (!kOpen) go3s<4>(st, a, k, s);
                     break;
-                case 7: go3k<8, 2, kOpen>(st, a, s); break;
+                case 7:
+                    if constexpr (kStaged) go_split<3, kOpen>(st, a, s);
+                    break;
                 case 8: go3k<8, 3, kOpen>(st, a, s); break;
                 case 9:
                     if constexpr (!kOpen) go3s<8, false>(st, a, k, s);
@@ -308,6 +336,14 @@ struct Launch {
             }
         }
     }
+
+    // Launch variant of a new solver: the two-pass step where it exists.  Measured on a B200,
+    // FP32, us per step, against the best march at its best planes per block (variant 8):
+    // 32x48x32 13 / 19, 64x96x64 41 / 54, 97x131x83 with walls 143 / 160, 128x256x128 341 / 428,
+    // 256x512x256 2570 / 2920, 64x160x64 with inlet and outflow 117 / 217.
+    static int default_variant(const DevState& st) { return kStaged && st.g.dim == 3 ? 7 : 0; }
+    // whether a variant marches over `seg` planes or rows per block
+    static bool marches(const DevState& st, int variant) { return !(kStaged && st.g.dim == 3 && variant == 7); }
 
     static cudaError_t step(const DevState& st, long long k, cudaStream_t s) {
         const StepArgs<PR> a = args(st, k);
@@ -384,6 +420,8 @@ struct Launch {
         t.prepare = &prepare;
         t.release = &release;
         t.available = &available;
+        t.default_variant = &default_variant;
+        t.marches = &marches;
         t.args_bytes = sizeof(StepArgs<PR>);
         t.make_args = &make_args;
         t.step2_batch = &step2_batch;
