@@ -659,12 +659,14 @@ __device__ __forceinline__ void update_node(const StepArgs<PR>& a, const Codec<P
         TP go[Q], gp[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) gp[q] = gpost(q);
-        macroscopic<DIM, T>(PT, fpost, c, mu, dc, u, p, rho);
+        // one branch per warp: see all_in_range
+        const bool in = __all_sync(__activemask(), all_in_range<Q, 500>(fpost) && all_in_range<DIM, 200>(u));
+        macroscopic<DIM, T>(PT, fpost, c, mu, dc, u, p, rho, in);
         collide_g<DIM, TP>(PP, gp, c, dc, u, go);  // Allen-Cahn relaxation
         // g is stored before the f collision, so its 19 values are not live through it
 #pragma unroll
         for (int q = 0; q < Q; ++q) cd.store_dev(a.gout + (self + unsigned(q) * unsigned(g.ps)), go[q]);
-        collide_f<DIM, T>(PT, fpost, c, mu, dc, rho, p, u, fo);  // force-corrected WMRT relaxation
+        collide_f<DIM, T>(PT, fpost, c, mu, dc, rho, p, u, fo, in);  // force-corrected WMRT relaxation
 #pragma unroll
         for (int q = 0; q < Q; ++q) cd.store_f(a.fout + (self + unsigned(q) * unsigned(g.ps)), fo[q]);
     } else {

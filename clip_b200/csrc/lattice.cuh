@@ -140,6 +140,95 @@ __device__ __forceinline__ T usq(T ux, T uy, T uz) {
     return DIM == 2 ? ux * ux + uy * uy : ux * ux + uy * uy + uz * uz;
 }
 
+// The same for every direction, with a pair's shared terms formed once: the opposite direction
+// has -e.u, whose products are the negated ones exactly.
+template <int DIM, typename T>
+__device__ __forceinline__ void equilibria(T ux, T uy, T uz, T U2, T* eq) {
+    using L = Lat<DIM>;
+    const T t3 = T(1.5) * U2;
+#pragma unroll
+    for (int q = 0; q < L::Q; ++q) {
+        const int o = opposite<DIM>(q);
+        if (o < q) continue;
+        const T eU = edot<DIM, T>(q, ux, uy, uz);
+        const T t1 = T(3.0) * eU, t2 = T(4.5) * eU * eU;
+        eq[q] = T(L::w(q)) * (t1 + t2 - t3);
+        if (o != q) eq[o] = T(L::w(o)) * (-t1 + t2 - t3);
+    }
+}
+
+// ---------------------------------------------------------------- FP64 quotients
+// The FP64 3D step has 69 quotients per node (the inverse transform's by 6, 36, 72, 144 and those
+// by rho); as general divisions they and their range checks were over half of its 8,800
+// instructions.  With these forms and the pairs' shared terms the 128x256x128 step went from
+// 1390 to 1082 us (32 x 16 tile), the 256x1024 2D step from 53 to 33 us.  Both forms below
+// return the correctly rounded quotient, the bits of a / b, for operands whose products stay
+// clear of underflow and overflow; callers check that with in_range and divide otherwise.
+//
+// By a constant D = 2^k 3^m, m <= 2: with hi + lo = 1/D to twice the precision, x hi + x lo is
+// off the quotient by less than 2^-50 of a unit in the last place before its one rounding, while
+// a quotient that is not itself a double lies at least 1/18 of a unit from every midpoint of
+// two doubles (2N - 9(2k + 1) is odd).  Method: Brisebarre, Muller, Raina, "Accelerating
+// correctly rounded floating-point division when the divisor is known in advance" (2004).
+template <int D>
+struct Reciprocal {
+    static constexpr double hi = 1.0 / D;
+    static constexpr double rest() {  // (1 - D hi) / D, the difference exact by splitting hi
+        const double t = 134217729.0 * hi, a = t - (t - hi), b = hi - a;
+        return ((1.0 - D * a) - D * b) / D;
+    }
+    static constexpr double lo = rest();
+};
+template <int D>
+__device__ __forceinline__ double divide_by(double x) {
+    return __fma_rn(x, Reciprocal<D>::hi, __dmul_rn(x, Reciprocal<D>::lo));
+}
+// a / b with y = 1 / b correctly rounded: the first correction makes the quotient faithful, the
+// second rounds it correctly (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990, theorem on division).
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+// x is zero or has 2^-E <= |x| < 2^E.
+template <int E>
+__device__ __forceinline__ bool in_range(double x) {
+    const unsigned t = unsigned(__double2hiint(x)) & 0x7fffffffu;
+    return t - (unsigned(1023 - E) << 20) < (unsigned(2 * E) << 20) || x == 0.0;
+}
+// The update's quotients may take these forms when every f is zero or within 2^+-500, every
+// velocity component zero or within 2^+-200, and (for the collision, and for the quotients of
+// the force itself) every force component zero or within 2^+-500: sums of such values are
+// zero or multiples of the units of their terms, above 2^-700, and the products with the
+// weights, the rates and the transforms' integers keep them above 2^-950.  The narrow tails in
+// which a field first spreads fall below, and non-finite values above.
+template <int N, int E, typename T>
+__device__ __forceinline__ bool all_in_range(const T* v) {
+    if constexpr (std::is_same<T, double>::value) {
+        bool ok = true;
+#pragma unroll
+        for (int i = 0; i < N; ++i) ok = ok && in_range<E>(v[i]);
+        return ok;
+    } else {
+        return false;
+    }
+}
+// a[i] / b for N values
+template <int N, typename T>
+__device__ __forceinline__ void divide_all(T* a, T b, bool in) {
+    if constexpr (std::is_same<T, double>::value) {
+        if (in && in_range<100>(b)) {
+            const double y = 1.0 / b;
+#pragma unroll
+            for (int i = 0; i < N; ++i) a[i] = quotient(a[i], b, y);
+            return;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) a[i] = a[i] / b;
+}
+
 // ---------------------------------------------------------------- WMRT (WMRT.cuh:54-184)
 template <typename T>
 __device__ __forceinline__ void wmrt_forward9(const T* in, T* out) {
@@ -155,19 +244,19 @@ __device__ __forceinline__ void wmrt_forward9(const T* in, T* out) {
     out[8] = in5 - in6 + in7 - in8;
 }
 
+// The inverse transforms without their divisors (36; wmrt_divisor19).
 template <typename T>
 __device__ __forceinline__ void wmrt_inverse9(const T* in, T* out) {
     const T in0 = in[0], in1 = in[1], in2 = in[2], in3 = in[3], in4 = in[4], in5 = in[5], in6 = in[6], in7 = in[7], in8 = in[8];
-    const T d = T(36.0);
-    out[0] = (T(4.0) * in0 - T(4.0) * in1 + T(4.0) * in2) / d;
-    out[1] = (T(4.0) * in0 - in1 - T(2.0) * in2 + T(6.0) * in3 - T(6.0) * in4 + T(9.0) * in7) / d;
-    out[2] = (T(4.0) * in0 - in1 - T(2.0) * in2 + T(6.0) * in5 - T(6.0) * in6 - T(9.0) * in7) / d;
-    out[3] = (T(4.0) * in0 - in1 - T(2.0) * in2 - T(6.0) * in3 + T(6.0) * in4 + T(9.0) * in7) / d;
-    out[4] = (T(4.0) * in0 - in1 - T(2.0) * in2 - T(6.0) * in5 + T(6.0) * in6 - T(9.0) * in7) / d;
-    out[5] = (T(4.0) * in0 + T(2.0) * in1 + in2 + T(6.0) * in3 + T(3.0) * in4 + T(6.0) * in5 + T(3.0) * in6 + T(9.0) * in8) / d;
-    out[6] = (T(4.0) * in0 + T(2.0) * in1 + in2 - T(6.0) * in3 - T(3.0) * in4 + T(6.0) * in5 + T(3.0) * in6 - T(9.0) * in8) / d;
-    out[7] = (T(4.0) * in0 + T(2.0) * in1 + in2 - T(6.0) * in3 - T(3.0) * in4 - T(6.0) * in5 - T(3.0) * in6 + T(9.0) * in8) / d;
-    out[8] = (T(4.0) * in0 + T(2.0) * in1 + in2 + T(6.0) * in3 + T(3.0) * in4 - T(6.0) * in5 - T(3.0) * in6 - T(9.0) * in8) / d;
+    out[0] = T(4.0) * in0 - T(4.0) * in1 + T(4.0) * in2;
+    out[1] = T(4.0) * in0 - in1 - T(2.0) * in2 + T(6.0) * in3 - T(6.0) * in4 + T(9.0) * in7;
+    out[2] = T(4.0) * in0 - in1 - T(2.0) * in2 + T(6.0) * in5 - T(6.0) * in6 - T(9.0) * in7;
+    out[3] = T(4.0) * in0 - in1 - T(2.0) * in2 - T(6.0) * in3 + T(6.0) * in4 + T(9.0) * in7;
+    out[4] = T(4.0) * in0 - in1 - T(2.0) * in2 - T(6.0) * in5 + T(6.0) * in6 - T(9.0) * in7;
+    out[5] = T(4.0) * in0 + T(2.0) * in1 + in2 + T(6.0) * in3 + T(3.0) * in4 + T(6.0) * in5 + T(3.0) * in6 + T(9.0) * in8;
+    out[6] = T(4.0) * in0 + T(2.0) * in1 + in2 - T(6.0) * in3 - T(3.0) * in4 + T(6.0) * in5 + T(3.0) * in6 - T(9.0) * in8;
+    out[7] = T(4.0) * in0 + T(2.0) * in1 + in2 - T(6.0) * in3 - T(3.0) * in4 - T(6.0) * in5 - T(3.0) * in6 + T(9.0) * in8;
+    out[8] = T(4.0) * in0 + T(2.0) * in1 + in2 + T(6.0) * in3 + T(3.0) * in4 - T(6.0) * in5 - T(3.0) * in6 - T(9.0) * in8;
 }
 
 template <typename T>
@@ -204,33 +293,35 @@ __device__ __forceinline__ void wmrt_inverse19(const T* in, T* out) {
     const T in0 = in[0], in1 = in[1], in2 = in[2], in3 = in[3], in4 = in[4], in5 = in[5], in6 = in[6], in7 = in[7],
             in8 = in[8], in9 = in[9], in10 = in[10], in11 = in[11], in12 = in[12], in13 = in[13], in14 = in[14],
             in15 = in[15], in16 = in[16], in17 = in[17], in18 = in[18];
-    const T d6 = T(6.0), d36 = T(36.0), d72 = T(72.0), d144 = T(144.0);
-    out[0] = (T(2.0) * in0 - T(3.0) * in9 + in16) / d6;
-    out[1] = (T(2.0) * in0 + T(6.0) * in1 + T(3.0) * in7 - T(6.0) * in10 - T(2.0) * in16 - T(3.0) * in17) / d36;
-    out[2] = (T(2.0) * in0 - T(6.0) * in1 + T(3.0) * in7 + T(6.0) * in10 - T(2.0) * in16 - T(3.0) * in17) / d36;
-    out[3] = (T(4.0) * in0 + T(12.0) * in2 - T(3.0) * in7 + T(9.0) * in8 - T(12.0) * in11 - T(4.0) * in16 + T(3.0) * in17 - T(9.0) * in18) / d72;
-    out[4] = (T(4.0) * in0 - T(12.0) * in2 - T(3.0) * in7 + T(9.0) * in8 + T(12.0) * in11 - T(4.0) * in16 + T(3.0) * in17 - T(9.0) * in18) / d72;
-    out[5] = (T(4.0) * in0 + T(12.0) * in3 - T(3.0) * in7 - T(9.0) * in8 - T(12.0) * in12 - T(4.0) * in16 + T(3.0) * in17 + T(9.0) * in18) / d72;
-    out[6] = (T(4.0) * in0 - T(12.0) * in3 - T(3.0) * in7 - T(9.0) * in8 + T(12.0) * in12 - T(4.0) * in16 + T(3.0) * in17 + T(9.0) * in18) / d72;
-    out[7] = (T(4.0) * in0 + T(12.0) * in1 + T(12.0) * in2 + T(36.0) * in4 + T(3.0) * in7 + T(9.0) * in8 + T(6.0) * in9 + T(6.0) * in10 + T(6.0) * in11 + T(18.0) * in13 - T(18.0) * in14 + T(2.0) * in16 + T(3.0) * in17 + T(9.0) * in18) / d144;
-    out[8] = (T(4.0) * in0 - T(12.0) * in1 - T(12.0) * in2 + T(36.0) * in4 + T(3.0) * in7 + T(9.0) * in8 + T(6.0) * in9 - T(6.0) * in10 - T(6.0) * in11 - T(18.0) * in13 + T(18.0) * in14 + T(2.0) * in16 + T(3.0) * in17 + T(9.0) * in18) / d144;
-    out[9] = (T(4.0) * in0 + T(12.0) * in1 - T(12.0) * in2 - T(36.0) * in4 + T(3.0) * in7 + T(9.0) * in8 + T(6.0) * in9 + T(6.0) * in10 - T(6.0) * in11 + T(18.0) * in13 + T(18.0) * in14 + T(2.0) * in16 + T(3.0) * in17 + T(9.0) * in18) / d144;
-    out[10] = (T(4.0) * in0 - T(12.0) * in1 + T(12.0) * in2 - T(36.0) * in4 + T(3.0) * in7 + T(9.0) * in8 + T(6.0) * in9 - T(6.0) * in10 + T(6.0) * in11 - T(18.0) * in13 - T(18.0) * in14 + T(2.0) * in16 + T(3.0) * in17 + T(9.0) * in18) / d144;
-    out[11] = (T(4.0) * in0 + T(12.0) * in1 + T(12.0) * in3 + T(36.0) * in6 + T(3.0) * in7 - T(9.0) * in8 + T(6.0) * in9 + T(6.0) * in10 + T(6.0) * in12 - T(18.0) * in13 + T(18.0) * in15 + T(2.0) * in16 + T(3.0) * in17 - T(9.0) * in18) / d144;
-    out[12] = (T(4.0) * in0 - T(12.0) * in1 - T(12.0) * in3 + T(36.0) * in6 + T(3.0) * in7 - T(9.0) * in8 + T(6.0) * in9 - T(6.0) * in10 - T(6.0) * in12 + T(18.0) * in13 - T(18.0) * in15 + T(2.0) * in16 + T(3.0) * in17 - T(9.0) * in18) / d144;
-    out[13] = (T(4.0) * in0 + T(12.0) * in1 - T(12.0) * in3 - T(36.0) * in6 + T(3.0) * in7 - T(9.0) * in8 + T(6.0) * in9 + T(6.0) * in10 - T(6.0) * in12 - T(18.0) * in13 - T(18.0) * in15 + T(2.0) * in16 + T(3.0) * in17 - T(9.0) * in18) / d144;
-    out[14] = (T(4.0) * in0 - T(12.0) * in1 + T(12.0) * in3 - T(36.0) * in6 + T(3.0) * in7 - T(9.0) * in8 + T(6.0) * in9 - T(6.0) * in10 + T(6.0) * in12 + T(18.0) * in13 + T(18.0) * in15 + T(2.0) * in16 + T(3.0) * in17 - T(9.0) * in18) / d144;
-    out[15] = (T(4.0) * in0 + T(12.0) * in2 + T(12.0) * in3 + T(36.0) * in5 - T(6.0) * in7 + T(6.0) * in9 + T(6.0) * in11 + T(6.0) * in12 + T(18.0) * in14 - T(18.0) * in15 + T(2.0) * in16 - T(6.0) * in17) / d144;
-    out[16] = (T(4.0) * in0 - T(12.0) * in2 - T(12.0) * in3 + T(36.0) * in5 - T(6.0) * in7 + T(6.0) * in9 - T(6.0) * in11 - T(6.0) * in12 - T(18.0) * in14 + T(18.0) * in15 + T(2.0) * in16 - T(6.0) * in17) / d144;
-    out[17] = (T(4.0) * in0 + T(12.0) * in2 - T(12.0) * in3 - T(36.0) * in5 - T(6.0) * in7 + T(6.0) * in9 + T(6.0) * in11 - T(6.0) * in12 + T(18.0) * in14 + T(18.0) * in15 + T(2.0) * in16 - T(6.0) * in17) / d144;
-    out[18] = (T(4.0) * in0 - T(12.0) * in2 + T(12.0) * in3 - T(36.0) * in5 - T(6.0) * in7 + T(6.0) * in9 - T(6.0) * in11 + T(6.0) * in12 - T(18.0) * in14 - T(18.0) * in15 + T(2.0) * in16 - T(6.0) * in17) / d144;
+    out[0] = T(2.0) * in0 - T(3.0) * in9 + in16;
+    out[1] = T(2.0) * in0 + T(6.0) * in1 + T(3.0) * in7 - T(6.0) * in10 - T(2.0) * in16 - T(3.0) * in17;
+    out[2] = T(2.0) * in0 - T(6.0) * in1 + T(3.0) * in7 + T(6.0) * in10 - T(2.0) * in16 - T(3.0) * in17;
+    out[3] = T(4.0) * in0 + T(12.0) * in2 - T(3.0) * in7 + T(9.0) * in8 - T(12.0) * in11 - T(4.0) * in16 + T(3.0) * in17 - T(9.0) * in18;
+    out[4] = T(4.0) * in0 - T(12.0) * in2 - T(3.0) * in7 + T(9.0) * in8 + T(12.0) * in11 - T(4.0) * in16 + T(3.0) * in17 - T(9.0) * in18;
+    out[5] = T(4.0) * in0 + T(12.0) * in3 - T(3.0) * in7 - T(9.0) * in8 - T(12.0) * in12 - T(4.0) * in16 + T(3.0) * in17 + T(9.0) * in18;
+    out[6] = T(4.0) * in0 - T(12.0) * in3 - T(3.0) * in7 - T(9.0) * in8 + T(12.0) * in12 - T(4.0) * in16 + T(3.0) * in17 + T(9.0) * in18;
+    out[7] = T(4.0) * in0 + T(12.0) * in1 + T(12.0) * in2 + T(36.0) * in4 + T(3.0) * in7 + T(9.0) * in8 + T(6.0) * in9 + T(6.0) * in10 + T(6.0) * in11 + T(18.0) * in13 - T(18.0) * in14 + T(2.0) * in16 + T(3.0) * in17 + T(9.0) * in18;
+    out[8] = T(4.0) * in0 - T(12.0) * in1 - T(12.0) * in2 + T(36.0) * in4 + T(3.0) * in7 + T(9.0) * in8 + T(6.0) * in9 - T(6.0) * in10 - T(6.0) * in11 - T(18.0) * in13 + T(18.0) * in14 + T(2.0) * in16 + T(3.0) * in17 + T(9.0) * in18;
+    out[9] = T(4.0) * in0 + T(12.0) * in1 - T(12.0) * in2 - T(36.0) * in4 + T(3.0) * in7 + T(9.0) * in8 + T(6.0) * in9 + T(6.0) * in10 - T(6.0) * in11 + T(18.0) * in13 + T(18.0) * in14 + T(2.0) * in16 + T(3.0) * in17 + T(9.0) * in18;
+    out[10] = T(4.0) * in0 - T(12.0) * in1 + T(12.0) * in2 - T(36.0) * in4 + T(3.0) * in7 + T(9.0) * in8 + T(6.0) * in9 - T(6.0) * in10 + T(6.0) * in11 - T(18.0) * in13 - T(18.0) * in14 + T(2.0) * in16 + T(3.0) * in17 + T(9.0) * in18;
+    out[11] = T(4.0) * in0 + T(12.0) * in1 + T(12.0) * in3 + T(36.0) * in6 + T(3.0) * in7 - T(9.0) * in8 + T(6.0) * in9 + T(6.0) * in10 + T(6.0) * in12 - T(18.0) * in13 + T(18.0) * in15 + T(2.0) * in16 + T(3.0) * in17 - T(9.0) * in18;
+    out[12] = T(4.0) * in0 - T(12.0) * in1 - T(12.0) * in3 + T(36.0) * in6 + T(3.0) * in7 - T(9.0) * in8 + T(6.0) * in9 - T(6.0) * in10 - T(6.0) * in12 + T(18.0) * in13 - T(18.0) * in15 + T(2.0) * in16 + T(3.0) * in17 - T(9.0) * in18;
+    out[13] = T(4.0) * in0 + T(12.0) * in1 - T(12.0) * in3 - T(36.0) * in6 + T(3.0) * in7 - T(9.0) * in8 + T(6.0) * in9 + T(6.0) * in10 - T(6.0) * in12 - T(18.0) * in13 - T(18.0) * in15 + T(2.0) * in16 + T(3.0) * in17 - T(9.0) * in18;
+    out[14] = T(4.0) * in0 - T(12.0) * in1 + T(12.0) * in3 - T(36.0) * in6 + T(3.0) * in7 - T(9.0) * in8 + T(6.0) * in9 - T(6.0) * in10 + T(6.0) * in12 + T(18.0) * in13 + T(18.0) * in15 + T(2.0) * in16 + T(3.0) * in17 - T(9.0) * in18;
+    out[15] = T(4.0) * in0 + T(12.0) * in2 + T(12.0) * in3 + T(36.0) * in5 - T(6.0) * in7 + T(6.0) * in9 + T(6.0) * in11 + T(6.0) * in12 + T(18.0) * in14 - T(18.0) * in15 + T(2.0) * in16 - T(6.0) * in17;
+    out[16] = T(4.0) * in0 - T(12.0) * in2 - T(12.0) * in3 + T(36.0) * in5 - T(6.0) * in7 + T(6.0) * in9 - T(6.0) * in11 - T(6.0) * in12 - T(18.0) * in14 + T(18.0) * in15 + T(2.0) * in16 - T(6.0) * in17;
+    out[17] = T(4.0) * in0 + T(12.0) * in2 - T(12.0) * in3 - T(36.0) * in5 - T(6.0) * in7 + T(6.0) * in9 + T(6.0) * in11 - T(6.0) * in12 + T(18.0) * in14 + T(18.0) * in15 + T(2.0) * in16 - T(6.0) * in17;
+    out[18] = T(4.0) * in0 - T(12.0) * in2 + T(12.0) * in3 - T(36.0) * in5 - T(6.0) * in7 + T(6.0) * in9 - T(6.0) * in11 + T(6.0) * in12 - T(18.0) * in14 - T(18.0) * in15 + T(2.0) * in16 - T(6.0) * in17;
 }
+__host__ __device__ constexpr int wmrt_divisor19(int q) { return q == 0 ? 6 : (q < 3 ? 36 : (q < 7 ? 72 : 144)); }
 
 // Relax the viscous moments (2D: 7,8; 3D: 4..8) by s, all others at rate 1
-// (NsAllen.cu:416-431, 435-454): gneq <- M^-1 S M gneq.
+// (NsAllen.cu:416-431, 435-454): gneq <- M^-1 S M gneq.  in: the quotients may take their short
+// forms (all_in_range).
 template <int DIM, typename T>
-__device__ __forceinline__ void wmrt_relax(T* gneq, T s) {
-    T m[Lat<DIM>::Q];
+__device__ __forceinline__ void wmrt_relax(T* gneq, T s, bool in) {
+    constexpr int Q = Lat<DIM>::Q;
+    T m[Q];
     if (DIM == 2) {
         wmrt_forward9<T>(gneq, m);
         m[7] = m[7] * s;
@@ -245,6 +336,25 @@ __device__ __forceinline__ void wmrt_relax(T* gneq, T s) {
         m[8] = m[8] * s;
         wmrt_inverse19<T>(m, gneq);
     }
+    if constexpr (std::is_same<T, double>::value) {
+        if (in) {
+            if constexpr (DIM == 2) {
+#pragma unroll
+                for (int q = 0; q < Q; ++q) gneq[q] = divide_by<36>(gneq[q]);
+            } else {
+                gneq[0] = divide_by<6>(gneq[0]);
+#pragma unroll
+                for (int q = 1; q < 3; ++q) gneq[q] = divide_by<36>(gneq[q]);
+#pragma unroll
+                for (int q = 3; q < 7; ++q) gneq[q] = divide_by<72>(gneq[q]);
+#pragma unroll
+                for (int q = 7; q < Q; ++q) gneq[q] = divide_by<144>(gneq[q]);
+            }
+            return;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) gneq[q] = gneq[q] / T(DIM == 2 ? 36.0 : double(wmrt_divisor19(q)));
 }
 
 // ---------------------------------------------------------------- scalar physics
@@ -315,16 +425,16 @@ __device__ __forceinline__ void viscous_force(const Phys<T>& P, const T* gneq, T
 // Total force mu grad c - p (rhoH-rhoL)/3 grad c + F_visc + F_gravity (NsAllen.cu:476-485).
 template <int DIM, typename T>
 __device__ __forceinline__ void total_force(const Phys<T>& P, const T* fpost, T p, T ux, T uy, T uz, T tau, T s9,
-                                            T mu, T rho, const T* dc, T* F) {
+                                            T mu, T rho, const T* dc, T* F, bool in) {
     using L = Lat<DIM>;
-    T gneq[L::Q];
-    const T U2 = usq<DIM, T>(ux, uy, uz);
+    T gneq[L::Q], eq[L::Q];
+    equilibria<DIM, T>(ux, uy, uz, usq<DIM, T>(ux, uy, uz), eq);
 #pragma unroll
     for (int q = 0; q < L::Q; ++q) {
-        const T geq = p * T(L::w(q)) + equilibrium<DIM, T>(q, ux, uy, uz, U2);
+        const T geq = p * T(L::w(q)) + eq[q];
         gneq[q] = fpost[q] - geq;
     }
-    wmrt_relax<DIM, T>(gneq, s9);
+    wmrt_relax<DIM, T>(gneq, s9, in);
     T fv[3];
     viscous_force<DIM, T>(P, gneq, tau, dc[0], dc[1], DIM == 3 ? dc[2] : T(0), fv);
 #pragma unroll
@@ -337,9 +447,10 @@ __device__ __forceinline__ void total_force(const Phys<T>& P, const T* fpost, T 
 // kernelMacroscopicg + kernelMacroscopicf at one node (NsAllen.cu:369-540).
 //   in : fpost (streamed, bounced), c, mu, dc of this step, u (previous step)
 //   out: u (this step), p, rho
+//   in: fpost (2^+-500) and u (2^+-200) are all_in_range
 template <int DIM, typename T>
 __device__ __forceinline__ void macroscopic(const Phys<T>& P, const T* fpost, T c, T mu, const T* dc, T* u, T& p_out,
-                                            T& rho_out) {
+                                            T& rho_out, bool in = false) {
     using L = Lat<DIM>;
     constexpr int Q = L::Q;
     const T rho = (P.RhoL + (c * P.drho));  // NsAllen.cu:538
@@ -349,7 +460,11 @@ __device__ __forceinline__ void macroscopic(const Phys<T>& P, const T* fpost, T 
     const T tau = relax_tau<T>(P, c);
     const T s9 = T(1.0) / (tau + T(0.50));
     T F[3];
-    total_force<DIM, T>(P, fpost, p, u[0], u[1], DIM == 3 ? u[2] : T(0), tau, s9, mu, rho, dc, F);
+    total_force<DIM, T>(P, fpost, p, u[0], u[1], DIM == 3 ? u[2] : T(0), tau, s9, mu, rho, dc, F, in);
+    T h[3] = {T(0), T(0), T(0)};
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) h[d] = T(0.50) * F[d];
+    divide_all<DIM, T>(h, rho, in && all_in_range<DIM, 500>(F));
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
         T s = T(0);
@@ -362,7 +477,7 @@ __device__ __forceinline__ void macroscopic(const Phys<T>& P, const T* fpost, T 
             s = first ? t : s + t;
             first = false;
         }
-        u[d] = s + T(0.50) * F[d] / rho;
+        u[d] = s + h[d];
     }
     p_out = p;
     rho_out = rho;
@@ -392,45 +507,63 @@ __device__ __forceinline__ void collide_g(const Phys<T>& P, const T* gpost, T c,
     interface_normal<DIM>(P, c, dc, nrm);
     const T cm = c - T(0.50);
     const T pref = ((P.amob3 * (T(1.0) - T(4.0) * (cm * cm))) / P.W);
+    T eq[Q];
+    equilibria<DIM, T>(ux, uy, uz, U2, eq);
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-        const T ga_wa = equilibrium<DIM, T>(q, ux, uy, uz, U2);
+        const int o = opposite<DIM>(q);
+        if (o < q) continue;
         const T eF = pref * edot<DIM, T>(q, nrm[0], nrm[1], DIM == 3 ? nrm[2] : T(0));
-        const T hlp = T(L::w(q)) * eF;
-        const T heq = c * (ga_wa + T(L::w(q))) + hlp;
-        gout[q] = gpost[q] * P.one_minus_wc + heq * P.wc;
+        const T hlp = T(L::w(q)) * eF;  // of the opposite direction: -hlp
+        gout[q] = gpost[q] * P.one_minus_wc + (c * (eq[q] + T(L::w(q))) + hlp) * P.wc;
+        if (o != q) gout[o] = gpost[o] * P.one_minus_wc + (c * (eq[o] + T(L::w(q))) - hlp) * P.wc;
     }
 }
 
 // kernelCollisionMRTf at one node (NsAllen.cu:589-763): force-corrected WMRT relaxation
 // with this step's p, c, mu, grad c, rho and u.
+// in: as for macroscopic (fpost).
 template <int DIM, typename T>
 __device__ __forceinline__ void collide_f(const Phys<T>& P, const T* fpost, T c, T mu, const T* dc, T rho, T p,
-                                          const T* u, T* fout) {
+                                          const T* u, T* fout, bool in = false) {
     using L = Lat<DIM>;
-    constexpr int Q = L::Q;
+    constexpr int Q = L::Q, H = (Q - 1) / 2;
     const T ux = u[0], uy = u[1], uz = DIM == 3 ? u[2] : T(0);
-    const T U2 = usq<DIM, T>(ux, uy, uz);
     const T tau = relax_tau<T>(P, c);
     const T s9 = T(1.0) / (tau + T(0.50));
-    {
-        T F[3];
-        total_force<DIM, T>(P, fpost, p, ux, uy, uz, tau, s9, mu, rho, dc, F);
-        T gneq[Q];
+    in = in && all_in_range<DIM, 200>(u);
+    T F[3];
+    total_force<DIM, T>(P, fpost, p, ux, uy, uz, tau, s9, mu, rho, dc, F, in);
+    in = in && all_in_range<DIM, 500>(F);
+    // hlp_q = 3 w_q e_q.F / rho of the first direction of each pair (the other's is -hlp_q)
+    T hlp[H];
+    int i = 0;
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const T eF = edot<DIM, T>(q, F[0], F[1], DIM == 3 ? F[2] : T(0));
-            const T hlp = T(3.0 * L::w(q)) * eF / rho;
-            const T feq = p * T(L::w(q)) + equilibrium<DIM, T>(q, ux, uy, uz, U2) - T(0.50) * hlp;
-            gneq[q] = fpost[q] - feq;
-        }
-        wmrt_relax<DIM, T>(gneq, s9);
+    for (int q = 1; q < Q; ++q)
+        if (opposite<DIM>(q) > q) hlp[i++] = T(3.0 * L::w(q)) * edot<DIM, T>(q, F[0], F[1], DIM == 3 ? F[2] : T(0));
+    divide_all<H, T>(hlp, rho, in);
+    T eq[Q], gneq[Q];
+    equilibria<DIM, T>(ux, uy, uz, usq<DIM, T>(ux, uy, uz), eq);
+    gneq[0] = fpost[0] - (p * T(L::w(0)) + eq[0]);
+    i = 0;
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const T eF = edot<DIM, T>(q, F[0], F[1], DIM == 3 ? F[2] : T(0));
-            const T hlp = T(3.0 * L::w(q)) * eF / rho;
-            fout[q] = fpost[q] - gneq[q] + hlp;
-        }
+    for (int q = 1; q < Q; ++q) {
+        const int o = opposite<DIM>(q);
+        if (o < q) continue;
+        const T half = T(0.50) * hlp[i++];
+        gneq[q] = fpost[q] - (p * T(L::w(q)) + eq[q] - half);
+        gneq[o] = fpost[o] - (p * T(L::w(q)) + eq[o] + half);
+    }
+    wmrt_relax<DIM, T>(gneq, s9, in);
+    fout[0] = fpost[0] - gneq[0];
+    i = 0;
+#pragma unroll
+    for (int q = 1; q < Q; ++q) {
+        const int o = opposite<DIM>(q);
+        if (o < q) continue;
+        const T h = hlp[i++];
+        fout[q] = fpost[q] - gneq[q] + h;
+        fout[o] = fpost[o] - gneq[o] - h;
     }
 }
 
