@@ -180,7 +180,7 @@ int clipb::solver_create(const CaseConfig& cfg, int precision, clipb_solver** ou
         }
     }
     if ((rc = s->alloc(&st.p, aux))) return rc;
-    if (c.dim == 3 && precision != CLIPB_FP64 && (rc = s->alloc(&st.cw, (size_t)g.ps * 8))) return rc;
+    if ((rc = s->alloc(&st.cw, (size_t)g.ps * 8))) return rc;
     if ((rc = s->alloc((void**)&st.c0, (size_t)g.ps * sizeof(double)))) return rc;
     st.red_blocks = 8 * 148;  // monitor blocks: a fixed count keeps the sums deterministic
     if ((rc = s->alloc((void**)&st.red, (size_t)2 * st.red_blocks * sizeof(double)))) return rc;

@@ -627,6 +627,40 @@ __device__ __forceinline__ void node_monitors(const StepArgs<PR>& a, typename PR
     mon[1] = 0.5 * (a.phys.RhoL + cs * a.phys.drho) * u2;
 }
 
+// The FP64 update of one node: macroscopic update, both collisions and the stores, in the
+// reference's operations.  pull() fills gp with the streamed g; it is called once u is known and
+// the new g is stored before the f collision, so that neither set of 19 is live through the
+// transforms.
+template <int DIM, class PR, class Pull>
+__device__ __forceinline__ void update_exact(const StepArgs<PR>& a, const Codec<PR>& cd, unsigned self,
+                                             const typename PR::T* fpost, Pull pull, const typename PR::TP* gp,
+                                             typename PR::TP c, typename PR::TP mu, const typename PR::TP* dc, double* mon) {
+    using T = typename PR::T;
+    constexpr int Q = Lat<DIM>::Q;
+    const Geom& g = a.g;
+    T u[3], p, rho;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) u[d] = a.uin[self + unsigned(d) * unsigned(g.ps)];
+    // one branch per warp: see all_in_range
+    const bool in = __all_sync(__activemask(), all_in_range<Q, 500>(fpost) && all_in_range<DIM, 200>(u));
+    macroscopic<DIM, T>(a.pt, fpost, c, mu, dc, u, p, rho, in);
+    {
+        T go[Q];
+        pull();
+        collide_g<DIM, T>(a.pp, gp, c, dc, u, go);  // Allen-Cahn relaxation
+#pragma unroll
+        for (int q = 0; q < Q; ++q) cd.store_dev(a.gout + (self + unsigned(q) * unsigned(g.ps)), go[q]);
+    }
+    T fo[Q];
+    collide_f<DIM, T>(a.pt, fpost, c, mu, dc, rho, p, u, fo, in);  // force-corrected WMRT relaxation
+#pragma unroll
+    for (int q = 0; q < Q; ++q) cd.store_f(a.fout + (self + unsigned(q) * unsigned(g.ps)), fo[q]);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) a.u[self + unsigned(d) * unsigned(g.ps)] = u[d];
+    a.cout[self] = c;
+    if (mon) node_monitors<DIM, PR>(a, c, u, mon);
+}
+
 // Macroscopic update and the next collision of one interior node, then its stores.
 //   fpost (T): streamed f;  gpost(q) (TP): streamed g as pull_g returns it;
 //   delta: sum of gpost(q) over q in ascending order (shifted storage only; the phase-field
@@ -647,38 +681,29 @@ __device__ __forceinline__ void update_node(const StepArgs<PR>& a, const Codec<P
     using A = typename PR::A;
     constexpr int Q = Lat<DIM>::Q;
     const Geom& g = a.g;
-    A* U = a.u;
-    T u[3];
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) u[d] = T(a.uin[self + unsigned(d) * unsigned(g.ps)]);
     if constexpr (PR::kExact) {
         (void)c_old;
         (void)delta;
         (void)cdest;
-        T fo[Q], p, rho;
-        TP go[Q], gp[Q];
+        TP gp[Q];
+        auto pull = [&]() {
 #pragma unroll
-        for (int q = 0; q < Q; ++q) gp[q] = gpost(q);
-        // one branch per warp: see all_in_range
-        const bool in = __all_sync(__activemask(), all_in_range<Q, 500>(fpost) && all_in_range<DIM, 200>(u));
-        macroscopic<DIM, T>(PT, fpost, c, mu, dc, u, p, rho, in);
-        collide_g<DIM, TP>(PP, gp, c, dc, u, go);  // Allen-Cahn relaxation
-        // g is stored before the f collision, so its 19 values are not live through it
-#pragma unroll
-        for (int q = 0; q < Q; ++q) cd.store_dev(a.gout + (self + unsigned(q) * unsigned(g.ps)), go[q]);
-        collide_f<DIM, T>(PT, fpost, c, mu, dc, rho, p, u, fo, in);  // force-corrected WMRT relaxation
-#pragma unroll
-        for (int q = 0; q < Q; ++q) cd.store_f(a.fout + (self + unsigned(q) * unsigned(g.ps)), fo[q]);
+            for (int q = 0; q < Q; ++q) gp[q] = gpost(q);
+        };
+        update_exact<DIM, PR>(a, cd, self, fpost, pull, gp, c, mu, dc, mon);
     } else {
+        T u[3];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) u[d] = T(a.uin[self + unsigned(d) * unsigned(g.ps)]);
         lean_update<DIM>(PT, lean_moments<DIM>(fpost), gpost, delta, c_old, c, mu, dc, u, cdest, [&](int q, T fo, TP go) {
             cd.store_dev(a.gout + (self + unsigned(q) * unsigned(g.ps)), go);
             cd.store_f(a.fout + (self + unsigned(q) * unsigned(g.ps)), fo);
         });
-    }
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) U[self + unsigned(d) * unsigned(g.ps)] = A(u[d]);
-    a.cout[self] = A(c);
-    if (mon) node_monitors<DIM, PR>(a, A(c), u, mon);
+        for (int d = 0; d < DIM; ++d) a.u[self + unsigned(d) * unsigned(g.ps)] = A(u[d]);
+        a.cout[self] = A(c);
+        if (mon) node_monitors<DIM, PR>(a, A(c), u, mon);
+    }
 }
 
 // Sum of the Q pulled values in ascending q (the order of ring_c and of lean_update's delta).

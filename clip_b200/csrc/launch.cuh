@@ -261,27 +261,38 @@ struct Launch {
     // The two-pass step (kernels_split.cuh).
     template <int DIM, bool kOpen>
     static void go_split(const DevState& st, const StepArgs<PR>& a, cudaStream_t s) {
+        using L = Lat<DIM>;
         const Geom& g = st.g;
-        const int nx = (g.n[0] + 31) / 32;
-        const int z0 = DIM == 3 ? g.zlo - 1 : 0, nz = DIM == 3 ? g.zhi - g.zlo + 1 : 1;
-        if constexpr (DIM == 3 && !kOpen && !PR::kExact) {
-            using L = Lat<3>;
-            PullPtrs<PR> ptr;
-            for (int q = 0; q < L::Q; ++q) {
-                const long long from = q * g.ps - L::ex(q) - L::ey(q) * g.sy - L::ez(q) * g.sz;
-                ptr.f[q] = a.fin + from;
-                ptr.g[q] = a.gin + from;
-                ptr.fo[q] = a.fout + q * g.ps;
-                ptr.go[q] = a.gout + q * g.ps;
+        PullPtrs<DIM, PR> ptr;
+        for (int q = 0; q < L::Q; ++q) {
+            const long long from = q * g.ps - L::ex(q) - L::ey(q) * g.sy - (DIM == 3 ? L::ez(q) * g.sz : 0);
+            ptr.f[q] = a.fin + from;
+            ptr.g[q] = a.gin + from;
+            ptr.fo[q] = a.fout + q * g.ps;
+            ptr.go[q] = a.gout + q * g.ps;
+        }
+        constexpr int TY = 4;
+        const int nx = (g.n[0] + 31) / 32, nz = DIM == 3 ? g.zhi - g.zlo + 1 : 1;
+        const int py = DIM == 3 ? 8 : 4;  // rows per block of the phase field
+        (void)launch_chained(phase_kernel<DIM, PR, kOpen>, dim3(nx, (g.n[1] + 2 + py - 1) / py, DIM == 3 ? nz + 2 : 1), dim3(32, py),
+                             0, s, a, ptr, g.zlo - 1);
+        const dim3 gu(nx, (g.n[1] + TY - 1) / TY, nz), bu(32, TY);
+        if constexpr (PR::kExact || kOpen) {
+            if constexpr (DIM == 3 && !kOpen) {
+                if (a.mon) {
+                    (void)launch_chained(update_wide_kernel<DIM, PR, kOpen, true>, gu, bu, 0, s, a, ptr);
+                    return;
+                }
             }
-            constexpr int TY = 4;
-            const dim3 gu(nx, (g.n[1] + TY - 1) / TY, nz), bu(32, TY);
-            (void)launch_chained(phase3_kernel<PR>, dim3(nx, (g.n[1] + 2 + 7) / 8, nz + 2), dim3(32, 8), 0, s, a, ptr, z0);
-            if (a.mon) (void)launch_chained(update3_kernel<PR, TY, true>, gu, bu, 0, s, a, ptr, z0 + 1);
-            else (void)launch_chained(update3_kernel<PR, TY, false>, gu, bu, 0, s, a, ptr, z0 + 1);
+            (void)launch_chained(update_wide_kernel<DIM, PR, kOpen, false>, gu, bu, 0, s, a, ptr);
         } else {
-            phase_kernel<DIM, PR, kOpen><<<dim3(nx, (g.n[1] + 2 + 7) / 8, DIM == 3 ? nz + 2 : 1), dim3(32, 8), 0, s>>>(a, z0);
-            update_kernel<DIM, PR, kOpen><<<dim3(nx, (g.n[1] + 3) / 4, nz), dim3(32, 4), 0, s>>>(a);
+            if constexpr (DIM == 3) {
+                if (a.mon) {
+                    (void)launch_chained(update_kernel<DIM, PR, TY, true>, gu, bu, 0, s, a, ptr, g.zlo);
+                    return;
+                }
+            }
+            (void)launch_chained(update_kernel<DIM, PR, TY, false>, gu, bu, 0, s, a, ptr, g.zlo);
         }
     }
 
@@ -295,10 +306,11 @@ struct Launch {
 
     // Launch variants (tile shape, whether g of the next plane stays in registers); the
     // autotuner in capi.cu picks one per solver.  kKeepG2/kKeepG3 = false restricts a
-    // precision to the re-pulling variants (FP64: registers).
+    // precision to the re-pulling variants (FP64: registers).  The two-pass step is variant 3 in
+    // 2D, 4 in 3D FP64 and 7 in 3D FP32/FP16.
     // Variants 5 and 6 (FP32/FP16) are the staged step with 32 x 8 and 32 x 4 tiles.
-    // Variant 7 (FP32/FP16) is the two-pass step, variant 8 keeps the next plane's g in shared
-    // memory, with at least 3 resident 32 x 8 blocks per SM.
+    // Variant 8 (FP32/FP16) keeps the next plane's g in shared memory, with at least 3 resident
+    // 32 x 8 blocks per SM.
     // Variant 9 (FP32/FP16) is the staged step with g by bulk copies and f pulled from global
     // memory, at least 2 resident 32 x 8 blocks per SM.
     static constexpr int kVariants3 = kStaged ? 10 : 5, kVariants2 = 4;
@@ -311,7 +323,10 @@ struct Launch {
                 case 1: go3<32, 8, kKeepG3, kOpen>(st, a, s); break;
                 case 2: go3<32, 16, false, kOpen>(st, a, s); break;
                 case 3: go3<64, 8, false, kOpen>(st, a, s); break;
-                case 4: go3<32, 4, kKeepG3, kOpen>(st, a, s); break;
+                case 4:
+                    if constexpr (PR::kExact) go_split<3, kOpen>(st, a, s);
+                    else go3<32, 4, kKeepG3, kOpen>(st, a, s);
+                    break;
                 case 5:
                     if constexpr (!kOpen) go3s<8>(st, a, k, s);
                     break;
@@ -331,19 +346,23 @@ struct Launch {
             switch (st.variant) {
                 case 1: go2<32, kKeepG2, kOpen>(st, a, s); break;
                 case 2: go2<128, kKeepG2, kOpen>(st, a, s); break;
-                case 3: go2<64, false, kOpen>(st, a, s); break;
+                case 3: go_split<2, kOpen>(st, a, s); break;
                 default: go2<64, kKeepG2, kOpen>(st, a, s); break;
             }
         }
     }
 
-    // Launch variant of a new solver: the two-pass step where it exists.  Measured on a B200,
-    // FP32, us per step, against the best march at its best planes per block (variant 8):
-    // 32x48x32 13 / 19, 64x96x64 41 / 54, 97x131x83 with walls 143 / 160, 128x256x128 341 / 428,
-    // 256x512x256 2570 / 2920, 64x160x64 with inlet and outflow 117 / 217.
-    static int default_variant(const DevState& st) { return kStaged && st.g.dim == 3 ? 7 : 0; }
+    // Launch variant of a new solver: the two-pass step.  Measured on a B200, us per step, against
+    // the best of the marching variants at its best planes or rows per block:
+    //   3D FP32: 32x48x32 13 / 19, 64x96x64 41 / 54, 97x131x83 with walls 143 / 160, 128x256x128
+    //     341 / 428, 256x512x256 2570 / 2920, 64x160x64 with inlet and outflow 117 / 217
+    //   3D FP64: 32x48x32 20 / 26, 64x96x64 92 / 137, 128x256x128 887 / 1082, 256^3 3620 / 4160
+    //   2D FP32: 64x128 6.1 / 7.4, 201x777 10.6 / 14.2, 256x1024 12.5 / 14.9, 1024x4096 158 / 171
+    //   2D FP64: 64x128 6.7 / 8.7, 201x777 19 / 27, 256x1024 28 / 33, 1024x4096 493 / 524
+    static constexpr int kTwoPass3 = PR::kExact ? 4 : 7, kTwoPass2 = 3;
+    static int default_variant(const DevState& st) { return st.g.dim == 3 ? kTwoPass3 : kTwoPass2; }
     // whether a variant marches over `seg` planes or rows per block
-    static bool marches(const DevState& st, int variant) { return !(kStaged && st.g.dim == 3 && variant == 7); }
+    static bool marches(const DevState& st, int variant) { return variant != default_variant(st); }
 
     static cudaError_t step(const DevState& st, long long k, cudaStream_t s) {
         const StepArgs<PR> a = args(st, k);

@@ -1,6 +1,7 @@
-"""The two-pass 3D step (launch variant 7, the default of the FP32/FP16 paths) against the
-one-pass march: every node's arithmetic is the same, so the state must be identical, at sizes
-around its 32 x 4 tiles and for every kind of side, in which the boundary work differs."""
+"""The two-pass step (the default launch: variant 7 of the 3D FP32/FP16 paths, 4 of the 3D FP64
+path, 3 of the 2D paths) against the one-pass march: every node's arithmetic is the same, so the
+state must be identical, at sizes around its 32 x 4 tiles and for every kind of side, in which
+the boundary work differs."""
 import numpy as np
 import pytest
 
@@ -13,16 +14,19 @@ TYPES = {"p": ("periodic", "periodic"), "w": ("wall", "wall"), "s": ("slipwall",
 
 
 def _config(path, n, sides):
-    lines = ["case = drop", "finalStep = 10", f"N = [{n[0] + 2}, {n[1] + 2}, {n[2] + 2}]", "referenceLength = 6",
+    dim = len(n)
+    size = [v + 2 for v in n] if dim == 3 else [n[0], n[1], 1]
+    center = [n[a] / 2 + 0.9 - 0.2 * a for a in range(dim)] + [0.0] * (3 - dim)
+    lines = ["case = drop", "finalStep = 10", f"N = {size}", "referenceLength = 6",
              "We = 8", "Re = 40", "gravity = [0, -1e-06, 0]", "mobility = 0.02", "interfaceWidth = 4", "muRatio = 10",
-             "rhoRatio = 100", "geometry = [", "  {", '    type = "sphere"',
-             f"    center = [{n[0] / 2 + 0.9}, {n[1] / 2 + 0.7}, {n[2] / 2 + 0.4}]", "    radius = 3", "    id = 0", "  }", "]",
+             "rhoRatio = 100", "geometry = [", "  {",
+             f'    type = "{"sphere" if dim == 3 else "circle"}"', f"    center = {center}", "    radius = 3", "    id = 0", "  }", "]",
              "boundary = ["]
     types = {"open": ["periodic", "periodic", "freeconvect", "velocity", "periodic", "periodic"],
              "inlet": ["periodic", "periodic", "wall", "velocity", "wall", "wall"]}.get(sides)
     if types is None:
         types = [t for s in sides for t in TYPES[s]]
-    for side, t in zip(("x-", "x+", "y-", "y+", "z-", "z+"), types):
+    for side, t in zip(("x-", "x+", "y-", "y+", "z-", "z+")[: 2 * dim], types):
         lines += ["  {", f'    side = "{side}"', f'    type = "{t}"']
         lines += ["    value = [0, -0.01, 0]"] if t == "velocity" else []
         lines += ["  },"]
@@ -40,17 +44,28 @@ def _run(path, prec, variant, steps, monitored):
         return {f: s.interior_field(f) for f in ("c", "vel", "f_post", "g_post")}, sums
 
 
-@pytest.mark.parametrize("prec", ["fp32", "fp16"])
-@pytest.mark.parametrize("n,sides", [((2, 2, 2), "ppp"), ((3, 5, 2), "ppp"), ((31, 4, 3), "pwp"), ((32, 8, 5), "pww"),
-                                     ((33, 9, 4), "wpp"), ((34, 3, 6), "www"), ((65, 7, 7), "ppp"), ((64, 13, 9), "spw"),
-                                     ((35, 11, 6), "inlet"), ((33, 10, 8), "open")])
-def test_two_pass_equals_the_march(tmp_path, prec, n, sides):
-    path = _config(tmp_path / "config.txt", n, sides)
+def _compare(path, prec, march, two_pass, monitored):
     # 19 steps: one 16-step graph and single launches
-    want, sums = _run(path, prec, 8, 19, sides != "open")
-    for variant in (7, None):
-        got, s2 = _run(path, prec, variant, 19, sides != "open")
+    want, sums = _run(path, prec, march, 19, monitored)
+    for variant in (two_pass, None):
+        got, s2 = _run(path, prec, variant, 19, monitored)
         for f in want:
             assert np.isfinite(got[f]).all()
             assert np.array_equal(got[f], want[f]), f
         assert s2 == sums
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32", "fp16"])
+@pytest.mark.parametrize("n,sides", [((2, 2, 2), "ppp"), ((3, 5, 2), "ppp"), ((31, 4, 3), "pwp"), ((32, 8, 5), "pww"),
+                                     ((33, 9, 4), "wpp"), ((34, 3, 6), "www"), ((65, 7, 7), "ppp"), ((64, 13, 9), "spw"),
+                                     ((35, 11, 6), "inlet"), ((33, 10, 8), "open")])
+def test_two_pass_equals_the_march_3d(tmp_path, prec, n, sides):
+    path = _config(tmp_path / "config.txt", n, sides)
+    _compare(path, prec, 2 if prec == "fp64" else 8, 4 if prec == "fp64" else 7, sides != "open")
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32", "fp16"])
+@pytest.mark.parametrize("n,sides", [((2, 2), "pp"), ((3, 5), "pw"), ((31, 4), "wp"), ((32, 8), "ww"), ((33, 9), "pp"),
+                                     ((64, 3), "sp"), ((65, 13), "pw"), ((35, 11), "inlet"), ((33, 10), "open")])
+def test_two_pass_equals_the_march_2d(tmp_path, prec, n, sides):
+    _compare(_config(tmp_path / "config.txt", n, sides), prec, 0, 3, False)
