@@ -1,5 +1,6 @@
-// Batched 2D cases (C ABI in include/clipb.h): many independent small cases advanced by one
-// persistent launch per time step (step2d_batch_kernel), replayed from a CUDA graph.  Each
+// Batched 2D cases (C ABI in include/clipb.h): many independent small cases advanced together,
+// by two launches per time step (phase_batch_kernel, update_batch_kernel; FP32/FP16) or one
+// persistent launch (step2d_batch_kernel), replayed from a CUDA graph.  Each
 // case is an ordinary solver (its own buffers, geometry and physics); the batch keeps a
 // device table of every case's step arguments for both buffer parities and a list of work
 // items (case, tile, row segment) built for the current launch shape.
@@ -183,6 +184,10 @@ int clipb_batch_create(const char* const* configs, int ncases, int kind, int pre
         s->stream = b->stream;  // every case runs on the batch's stream
     }
     b->kt = b->cases[0]->kt;
+    if (precision != CLIPB_FP64) {  // the two-pass step (its rates: update_batch_kernel)
+        b->variant = b->kt.default_variant(b->cases[0]->st);
+        b->seg = 16;
+    }
     // step arguments of every case for both buffer parities
     const size_t ab = b->kt.args_bytes;
     std::vector<unsigned char> host(ab * ncases);
@@ -323,6 +328,7 @@ int clipb_batch_autotune(clipb_batch* b, int trial_steps, int* best_variant, int
         if (!b->kt.available(b->cases[0]->st, v)) continue;
         for (int seg : {4, 8, 16, 32, 64})
             for (int bps : {1, 2, 0}) {
+                if (bps && b->precision != CLIPB_FP64 && !b->kt.marches(b->cases[0]->st, v)) continue;  // not persistent
                 if ((rc = clipb_batch_set_launch(b, v, seg, bps))) return rc;
                 if ((rc = clipb_batch_solve(b, 1))) return rc;  // warm-up
                 float ms = 0.f;

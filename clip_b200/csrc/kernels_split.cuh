@@ -33,6 +33,20 @@ struct PullPtrs {
     const typename PR::Sg* g[Lat<DIM>::Q];
     typename PR::Sf* fo[Lat<DIM>::Q];
     typename PR::Sg* go[Lat<DIM>::Q];
+    __device__ __forceinline__ const typename PR::Sf* f_from(int q, unsigned i) const { return f[q] + i; }
+    __device__ __forceinline__ const typename PR::Sg* g_from(int q, unsigned i) const { return g[q] + i; }
+    __device__ __forceinline__ typename PR::Sf* f_to(int q, unsigned i) const { return fo[q] + i; }
+    __device__ __forceinline__ typename PR::Sg* g_to(int q, unsigned i) const { return go[q] + i; }
+};
+// The same from the buffers' bases, for the cases of a batch, whose arguments are not kernel
+// parameters.
+template <int DIM, class PR>
+struct BasePtrs {
+    const StepArgs<PR>& a;
+    __device__ __forceinline__ const typename PR::Sf* f_from(int q, unsigned i) const { return a.fin + (i + pull_offset<DIM>(a.g, q)); }
+    __device__ __forceinline__ const typename PR::Sg* g_from(int q, unsigned i) const { return a.gin + (i + pull_offset<DIM>(a.g, q)); }
+    __device__ __forceinline__ typename PR::Sf* f_to(int q, unsigned i) const { return a.fout + (i + unsigned(q) * unsigned(a.g.ps)); }
+    __device__ __forceinline__ typename PR::Sg* g_to(int q, unsigned i) const { return a.gout + (i + unsigned(q) * unsigned(a.g.ps)); }
 };
 
 // Boundary summary of one node: element offsets that wrap a source beyond a periodic x side,
@@ -94,22 +108,15 @@ __device__ __forceinline__ void unshift(const Column<DIM>& col, const float* wc,
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// c of this step at (x, y, z), ghost coordinates included.  Bound by memory: 70 us on the
-// 128x256x128 bubble in FP32, 88 bytes per node at 5.3 TB/s (79 us, 382 instead of 230
-// instructions per node, with the general pull in every warp next to a side).
-template <int DIM, class PR, bool kOpen>
-__global__ void __launch_bounds__(256) phase_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr, int z_first) {
+// c of this step at (x, y, z), ghost coordinates included (x an interior node's: its neighbours
+// in the x ghost columns with it).
+template <int DIM, class PR, bool kOpen, class Ptr>
+__device__ __forceinline__ void phase_node(const StepArgs<PR>& a, const Ptr& ptr, int x, int y, int z) {
     using L = Lat<DIM>;
     using TP = typename PR::TP;
     using A = typename PR::A;
     const Geom& g = a.g;
     const Codec<PR> cd(a.pop_scale);
-    const int x = 1 + (int)(blockIdx.x * 32 + threadIdx.x), y = (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    const int z = DIM == 3 ? z_first + (int)blockIdx.z : 0;
-    // in this order: the update may start once everything before this kernel has ended
-    wait_for_predecessor();
-    let_successor_start();
-    if (x > g.n[0] || y > g.n[1] + 1) return;
     const unsigned self = nidx32(g, x, y, z);
     typename PR::Ring c;
     if (y >= 1 && y <= g.n[1] && (DIM == 2 || (z >= 1 && z <= g.n[2]))) {
@@ -120,7 +127,7 @@ __global__ void __launch_bounds__(256) phase_kernel(StepArgs<PR> a, PullPtrs<DIM
         } else {
             if constexpr (PR::kShift) cs = a.cin[self];
 #pragma unroll
-            for (int q = 0; q < L::Q; ++q) v[q] = cd.load_dev(ptr.g[q] + col.from(self, L::ex(q)));
+            for (int q = 0; q < L::Q; ++q) v[q] = cd.load_dev(ptr.g_from(q, col.from(self, L::ex(q))));
             if constexpr (PR::kShift)
                 if (col.wraps()) {
                     float wc[L::A];
@@ -137,6 +144,18 @@ __global__ void __launch_bounds__(256) phase_kernel(StepArgs<PR> a, PullPtrs<DIM
     if (x == g.n[0]) a.cw[self + 1] = ring_of<PR>(ghost_c<DIM, A>(a.cin, g, x + 1, y, z));
 }
 
+// Bound by memory: 70 us on the 128x256x128 bubble in FP32, 88 bytes per node at 5.3 TB/s (79
+// us, 382 instead of 230 instructions per node, with the general pull in every warp next to a
+// side).
+template <int DIM, class PR, bool kOpen>
+__global__ void __launch_bounds__(256) phase_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr, int z_first) {
+    const int x = 1 + (int)(blockIdx.x * 32 + threadIdx.x), y = (int)(blockIdx.y * blockDim.y + threadIdx.y);
+    // in this order: the update may start once everything before this kernel has ended
+    wait_for_predecessor();
+    let_successor_start();
+    if (x <= a.g.n[0] && y <= a.g.n[1] + 1) phase_node<DIM, PR, kOpen>(a, ptr, x, y, DIM == 3 ? z_first + (int)blockIdx.z : 0);
+}
+
 // 8 bytes from global to shared memory without a register between (completion: copy_async_wait
 // of the issuing thread, then a barrier).
 __device__ __forceinline__ void copy_async8(void* dst, const void* src) {
@@ -144,27 +163,17 @@ __device__ __forceinline__ void copy_async8(void* dst, const void* src) {
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// FP32/FP16 update of one node per thread, blocks of 32 x TY nodes of a plane, cases without
-// open sides.  In 3D bound by memory (340 bytes of DRAM traffic per node at 5.1 TB/s; a bare
-// copy of the same populations runs at 5.8).  A block asks for all populations of its nodes, u
-// and the old c before it waits for anything; f is reduced to its moments as it arrives, so
-// that 128 registers hold it all without spills (a spilled load in flight stalls: at 80
-// registers and 24 warps per SM the 128x256x128 update took 370 instead of 277 us).  Small
-// blocks of 4 rows keep the loads of some beside the arithmetic of others: 8 rows took 316 us,
-// 2 rows 277.
-template <int DIM, class PR, int TY, bool kMon>
-__global__ void __launch_bounds__(32 * TY, 16 / TY) update_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr, int z_first) {
+// FP32/FP16 update of the 32 x TY tile of a plane whose first node is (x0, y0, z), rows up to
+// y_last, one node per thread, cases without open sides.  PT: a.pt, PP: a.pp (or copies of them in registers).
+template <int DIM, class PR, int TY, bool kMon, class Ptr>
+__device__ __forceinline__ void update_tile(const StepArgs<PR>& a, const Phys<float>& PT, const Phys<float>& PP, const Ptr& ptr,
+                                            int x0, int y0, int z, int y_last, float2 (*tile)[TY + 2][34]) {
     using L = Lat<DIM>;
-    constexpr int Q = L::Q, CW = 34;  // tile row: the nodes x0 - 1 .. x0 + 32
-    constexpr int PZ = DIM == 3 ? 3 : 1;
-    __shared__ float2 tile[PZ][TY + 2][CW];
+    constexpr int Q = L::Q, PZ = DIM == 3 ? 3 : 1;
     const Geom& g = a.g;
     const Codec<PR> cd(a.pop_scale);
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = 1 + (int)blockIdx.x * 32, x = x0 + tx, y0 = (int)blockIdx.y * TY, y = 1 + y0 + ty;
-    // planes in descending order: phase_kernel left the g of the highest ones in L2
-    const int z = DIM == 3 ? z_first + (int)(gridDim.z - 1 - blockIdx.z) : 0;
-    const bool active = x <= g.n[0] && y <= g.n[1];
+    const int tx = threadIdx.x, ty = threadIdx.y, x = x0 + tx, y = y0 + ty;
+    const bool active = x <= g.n[0] && y <= y_last;
     const unsigned self = nidx32(g, x, y, z);
     const Column<DIM> col(g, x, y, z);
     const bool fast = !__any_sync(0xffffffffu, active && col.general);
@@ -172,23 +181,23 @@ __global__ void __launch_bounds__(32 * TY, 16 / TY) update_kernel(StepArgs<PR> a
     if (active) {
         if (fast) {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) f[q] = cd.load_f(ptr.f[q] + col.from(self, L::ex(q)));
+            for (int q = 0; q < Q; ++q) f[q] = cd.load_f(ptr.f_from(q, col.from(self, L::ex(q))));
 #pragma unroll
-            for (int q = 0; q < Q; ++q) d[q] = cd.load_dev(ptr.g[q] + col.from(self, L::ex(q)));
+            for (int q = 0; q < Q; ++q) d[q] = cd.load_dev(ptr.g_from(q, col.from(self, L::ex(q))));
             if (col.wraps()) wrapped_c<DIM>(a.cin, g, col, self, wc);
         }
         cold = a.cin[self];
 #pragma unroll
         for (int k = 0; k < DIM; ++k) u[k] = a.uin[self + unsigned(k) * unsigned(g.ps)];
     }
-    // c of the tile and the nodes around it: phase_kernel, which this launch may overlap up to
-    // here (the requests above read nothing it writes)
+    // c of the tile and the nodes around it (tile row: x0 - 1 .. x0 + 32), from the phase field,
+    // which this launch may overlap up to here (the requests above read nothing it writes)
     wait_for_predecessor();
     let_successor_start();
     for (int r = ty; r < PZ * (TY + 2); r += TY) {
         const int dz = DIM == 3 ? r / (TY + 2) : 0, dy = r - dz * (TY + 2);
-        if (y0 + dy > g.n[1] + 1) continue;
-        const float2* src = a.cw + nidx32(g, x - 1, y0 + dy, DIM == 3 ? z - 1 + dz : 0);
+        if (y0 + dy > g.n[1] + 2) continue;
+        const float2* src = a.cw + nidx32(g, x - 1, y0 - 1 + dy, DIM == 3 ? z - 1 + dz : 0);
         float2* dst = &tile[dz][dy][tx];
         if (x - 1 <= g.n[0] + 1) copy_async8(dst, src);
         if (tx < 2 && x + 31 <= g.n[0] + 1) copy_async8(dst + 32, src + 32);
@@ -209,23 +218,79 @@ __global__ void __launch_bounds__(32 * TY, 16 / TY) update_kernel(StepArgs<PR> a
     if (active) {
         auto C = [&](int dx, int dy, int dz) { return tile[PZ / 2 + dz][1 + ty + dy][1 + tx + dx]; };
         float mu, dc[3] = {0.f, 0.f, 0.f};
-        stencil_hilo<DIM>(a.pp, C, mu, dc);
+        stencil_hilo<DIM>(PP, C, mu, dc);
         const float c = C(0, 0, 0).x;
         const unsigned dmask = cross_mask<DIM, true>(g, x, y, z);
         auto cdest = [&](int q) {
             return dest_shift_q<DIM, PR>(q, dmask, c, [&](int dx, int dy, int dz) { return C(dx, dy, dz).x; });
         };
-        lean_update<DIM>(a.pt, m, [&](int q) { return d[q]; }, delta, cold, c, mu, dc, u, cdest,
-                         [&](int q, float fo, float go) {
-                             cd.store_dev(ptr.go[q] + self, go);
-                             cd.store_f(ptr.fo[q] + self, fo);
-                         });
+        lean_update<DIM>(PT, m, [&](int q) { return d[q]; }, delta, cold, c, mu, dc, u, cdest, [&](int q, float fo, float go) {
+            cd.store_dev(ptr.g_to(q, self), go);
+            cd.store_f(ptr.f_to(q, self), fo);
+        });
 #pragma unroll
         for (int k = 0; k < DIM; ++k) a.u[self + unsigned(k) * unsigned(g.ps)] = u[k];
         a.cout[self] = c;
         if constexpr (kMon) node_monitors<DIM, PR>(a, c, u, mon);
     }
     if constexpr (kMon) store_monitor_row(a, tx, x0, y, z, mon);
+}
+
+// In 3D bound by memory (340 bytes of DRAM traffic per node at 5.1 TB/s; a bare copy of the same
+// populations runs at 5.8).  A block asks for all populations of its nodes, u and the old c
+// before it waits for anything; f is reduced to its moments as it arrives, so that 128
+// registers hold it all without spills (a spilled load in flight stalls: at 80 registers and
+// 24 warps per SM the 128x256x128 update took 370 instead of 277 us).  Small blocks of 4 rows
+// keep the loads of some beside the arithmetic of others: 8 rows took 316 us, 2 rows 277.
+template <int DIM, class PR, int TY, bool kMon>
+__global__ void __launch_bounds__(32 * TY, 16 / TY) update_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr, int z_first) {
+    __shared__ float2 tile[DIM == 3 ? 3 : 1][TY + 2][34];
+    // planes in descending order: phase_kernel left the g of the highest ones in L2
+    update_tile<DIM, PR, TY, kMon>(a, a.pt, a.pp, ptr, 1 + (int)blockIdx.x * 32, 1 + (int)blockIdx.y * TY,
+                                   DIM == 3 ? z_first + (int)(gridDim.z - 1 - blockIdx.z) : 0, a.g.n[1], tile);
+}
+
+// The two passes over the cases of a batch (2D, FP32/FP16): a block takes one work item (case,
+// tile column bx, rows by * seg + 1 ... of it), its case's step arguments copied from the device
+// table into shared memory.  512 seeded-size cases (22.2 M nodes), FP32: 0.97 ms per step at 16
+// rows per item (4 rows 1.09, 8 1.00, 64 0.99) against 1.15 ms for the marching batch kernel.
+template <class PR>
+__device__ __forceinline__ void copy_args(StepArgs<PR>* sa, const StepArgs<PR>* args) {
+    static_assert(sizeof(StepArgs<PR>) % 4 == 0, "copied in 4-byte words");
+    const unsigned* src = reinterpret_cast<const unsigned*>(args);
+    unsigned* dst = reinterpret_cast<unsigned*>(sa);
+    for (int w = (int)(threadIdx.y * 32 + threadIdx.x); w < (int)(sizeof(StepArgs<PR>) / 4); w += (int)(32 * blockDim.y)) dst[w] = src[w];
+    __syncthreads();
+}
+template <class PR>
+__global__ void __launch_bounds__(128) phase_batch_kernel(const StepArgs<PR>* __restrict__ args, const int* __restrict__ items, int seg) {
+    __shared__ StepArgs<PR> a;
+    const int* it = items + 3 * blockIdx.x;
+    const int x = 1 + it[1] * 32 + (int)threadIdx.x, by = it[2];
+    copy_args(&a, args + it[0]);
+    wait_for_predecessor();
+    let_successor_start();
+    const int n1 = a.g.n[1], last = min(by * seg + seg, n1);
+    if (x > a.g.n[0]) return;
+    const BasePtrs<2, PR> ptr{a};
+    for (int y = (by == 0 ? 0 : by * seg + 1) + (int)threadIdx.y; y <= (last == n1 ? n1 + 1 : last); y += 4)
+        phase_node<2, PR, false>(a, ptr, x, y, 0);
+}
+template <class PR>
+__global__ void __launch_bounds__(128, 8) update_batch_kernel(const StepArgs<PR>* __restrict__ args, const int* __restrict__ items, int seg) {
+    __shared__ StepArgs<PR> a;
+    __shared__ float2 tile[1][6][34];
+    const int* it = items + 3 * blockIdx.x;
+    const int bx = it[1], by = it[2];
+    copy_args(&a, args + it[0]);
+    // the parameters as locals: through a reference to shared memory every use is a load
+    const Phys<float> PT = a.pt, PP = a.pp;
+    const BasePtrs<2, PR> ptr{a};
+    const int y1 = min(by * seg + seg, a.g.n[1]);
+    for (int y = by * seg + 1; y <= y1; y += 4) {
+        update_tile<2, PR, 4, false>(a, PT, PP, ptr, 1 + bx * 32, y, 0, y1, tile);
+        __syncthreads();  // the tile is reused by the next rows
+    }
 }
 
 // The same for FP64 and for cases with open sides, c read through L1.  FP64: bound by the FP64
@@ -250,7 +315,7 @@ __global__ void __launch_bounds__(128, 4) update_wide_kernel(StepArgs<PR> a, Pul
         T fpost[Q];
         if (fast) {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) fpost[q] = cd.load_f(ptr.f[q] + col.from(self, L::ex(q)));
+            for (int q = 0; q < Q; ++q) fpost[q] = cd.load_f(ptr.f_from(q, col.from(self, L::ex(q))));
         } else {
             pull_f<DIM, PR, kOpen>(a.fin, cd, g, x, y, z, self, mask, fpost, a.par);
         }
@@ -269,7 +334,7 @@ __global__ void __launch_bounds__(128, 4) update_wide_kernel(StepArgs<PR> a, Pul
         auto pull = [&]() {
             if (fast) {
 #pragma unroll
-                for (int q = 0; q < Q; ++q) gpost[q] = cd.load_dev(ptr.g[q] + col.from(self, L::ex(q)));
+                for (int q = 0; q < Q; ++q) gpost[q] = cd.load_dev(ptr.g_from(q, col.from(self, L::ex(q))));
             } else {
                 pull_g<DIM, PR, kOpen>(a.gin, a.cin, cd, g, x, y, z, self, mask, gpost, cold, a.par);
             }

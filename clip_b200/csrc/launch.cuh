@@ -224,11 +224,18 @@ struct Launch {
         switch (variant) {
             case 1: return go2_batch<32, kKeepG2>(args, items, nitems, seg, blocks_per_sm, s);
             case 2: return go2_batch<128, kKeepG2>(args, items, nitems, seg, blocks_per_sm, s);
-            case 3: return go2_batch<64, false>(args, items, nitems, seg, blocks_per_sm, s);
+            case 3:
+                if constexpr (PR::kExact) {
+                    return go2_batch<64, false>(args, items, nitems, seg, blocks_per_sm, s);
+                } else {
+                    const auto* table = static_cast<const StepArgs<PR>*>(args);
+                    const cudaError_t e = launch_chained(phase_batch_kernel<PR>, dim3(nitems), dim3(32, 4), 0, s, table, items, seg);
+                    return e != cudaSuccess ? e : launch_chained(update_batch_kernel<PR>, dim3(nitems), dim3(32, 4), 0, s, table, items, seg);
+                }
             default: return go2_batch<64, kKeepG2>(args, items, nitems, seg, blocks_per_sm, s);
         }
     }
-    static int tile2(int variant) { return variant == 1 ? 32 : (variant == 2 ? 128 : 64); }
+    static int tile2(int variant) { return variant == 1 || (!PR::kExact && variant == 3) ? 32 : (variant == 2 ? 128 : 64); }
     static void make_args(const DevState& st, long long k, void* out) {
         const StepArgs<PR> a = args(st, k);
         std::memcpy(out, &a, sizeof(a));

@@ -69,3 +69,19 @@ def test_two_pass_equals_the_march_3d(tmp_path, prec, n, sides):
                                      ((64, 3), "sp"), ((65, 13), "pw"), ((35, 11), "inlet"), ((33, 10), "open")])
 def test_two_pass_equals_the_march_2d(tmp_path, prec, n, sides):
     _compare(_config(tmp_path / "config.txt", n, sides), prec, 0, 3, False)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp16"])
+@pytest.mark.parametrize("rows", [1, 5, 16, 64])
+def test_two_pass_batch_equals_the_march(prec, rows):
+    """Rows per work item that the 4-row tiles do not divide, and items longer than a case."""
+    texts = [cb.seeded_case_config(31, i) for i in range(5)]
+    out = []
+    for variant, seg in ((1, 8), (3, rows)):
+        with cb.Batch(texts, prec, texts=True) as b:
+            b.set_launch(variant, seg)
+            b.init()
+            b.solve(19)
+            out.append([b.case(i).interior_field(f) for i in range(5) for f in ("c", "vel", "g")])
+    for a, b in zip(*out):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
