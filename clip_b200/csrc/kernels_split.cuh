@@ -293,19 +293,29 @@ __global__ void __launch_bounds__(128, 8) update_batch_kernel(const StepArgs<PR>
     }
 }
 
-// The same for FP64 and for cases with open sides, c read through L1.  FP64: bound by the FP64
-// pipe and the latency of its chains, 2,340 operations per 3D node; g is pulled once the new
-// velocity is known, so that its 19 values are not live through the force.  128 registers, 16
-// warps per SM (3D, 128x256x128: 1011 us with phase_kernel; at 168 registers 1017, at 96 1083).
+// Rows per block and blocks per SM of update_wide_kernel.  FP64: bound by the FP64 pipe (64% busy
+// in 3D, 2,340 operations per node), the latency of its chains and instruction fetch (3,400
+// instructions in a straight line, so that warps of one block, which run close together, share
+// fetches).  3D takes 16 warps per SM as two blocks (128x256x128: 876 us per step with
+// phase_kernel; four blocks of 4 rows 900, three with 168 registers 913, five 1039; three passes
+// of one loop over the transforms 911 to 935); 2D takes 20 warps (512x2048: 117 us, with 16 125).
+template <int DIM, class PR>
+struct WideShape {
+    static constexpr int kRows = PR::kExact && DIM == 3 ? 8 : 4;
+    static constexpr int kBlocks = PR::kExact ? (DIM == 3 ? 2 : 5) : 4;
+};
+// The same for FP64 and for cases with open sides, c read through L1.  FP64 pulls g once the new
+// velocity is known, so that its 19 values are not live through the force.
 template <int DIM, class PR, bool kOpen, bool kMon>
-__global__ void __launch_bounds__(128, 4) update_wide_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr) {
+__global__ void __launch_bounds__((32 * WideShape<DIM, PR>::kRows), (WideShape<DIM, PR>::kBlocks))
+    update_wide_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr) {
     using L = Lat<DIM>;
     using TP = typename PR::TP;
     using T = typename PR::T;
     constexpr int Q = L::Q;
     const Geom& g = a.g;
     const Codec<PR> cd(a.pop_scale);
-    const int tx = threadIdx.x, x0 = 1 + (int)blockIdx.x * 32, x = x0 + tx, y = 1 + (int)(blockIdx.y * 4 + threadIdx.y);
+    const int tx = threadIdx.x, x0 = 1 + (int)blockIdx.x * 32, x = x0 + tx, y = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
     const int z = DIM == 3 ? g.zlo + (int)(gridDim.z - 1 - blockIdx.z) : 0;
     double mon[2] = {0.0, 0.0};
     if (x <= g.n[0] && y <= g.n[1]) {

@@ -278,7 +278,7 @@ struct Launch {
             ptr.fo[q] = a.fout + q * g.ps;
             ptr.go[q] = a.gout + q * g.ps;
         }
-        constexpr int TY = 4;
+        constexpr int TY = PR::kExact || kOpen ? WideShape<DIM, PR>::kRows : 4;
         const int nx = (g.n[0] + 31) / 32, nz = DIM == 3 ? g.zhi - g.zlo + 1 : 1;
         const int py = DIM == 3 ? 8 : 4;  // rows per block of the phase field
         (void)launch_chained(phase_kernel<DIM, PR, kOpen>, dim3(nx, (g.n[1] + 2 + py - 1) / py, DIM == 3 ? nz + 2 : 1), dim3(32, py),
