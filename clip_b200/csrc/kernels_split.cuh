@@ -1,5 +1,5 @@
 // The step in two passes: the phase field c of every node first (phase_kernel, into the work
-// array StepArgs::cw), then the update of every node (update_kernel, update_exact_kernel), one
+// array StepArgs::cw), then the update of every node (update_kernel, update_fp64_kernel), one
 // thread per node.
 //
 // The one-pass kernels (step2d_body, step3d_body) compute c on a tile and its halo while they
@@ -122,7 +122,7 @@ __device__ __forceinline__ void phase_node(const StepArgs<PR>& a, const Ptr& ptr
     if (y >= 1 && y <= g.n[1] && (DIM == 2 || (z >= 1 && z <= g.n[2]))) {
         const Column<DIM> col(g, x, y, z);
         TP v[L::Q], cs = TP(0);
-        if (kOpen || __any_sync(__activemask(), col.general)) {
+        if (__any_sync(__activemask(), col.general)) {
             pull_g<DIM, PR, kOpen>(a.gin, a.cin, cd, g, x, y, z, self, cross_mask<DIM>(g, x, y, z), v, cs, a.par);
         } else {
             if constexpr (PR::kShift) cs = a.cin[self];
@@ -164,8 +164,8 @@ __device__ __forceinline__ void copy_async8(void* dst, const void* src) {
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // FP32/FP16 update of the 32 x TY tile of a plane whose first node is (x0, y0, z), rows up to
-// y_last, one node per thread, cases without open sides.  PT: a.pt, PP: a.pp (or copies of them in registers).
-template <int DIM, class PR, int TY, bool kMon, class Ptr>
+// y_last, one node per thread.  PT: a.pt, PP: a.pp (or copies of them in registers).
+template <int DIM, class PR, int TY, bool kOpen, bool kMon, class Ptr>
 __device__ __forceinline__ void update_tile(const StepArgs<PR>& a, const Phys<float>& PT, const Phys<float>& PP, const Ptr& ptr,
                                             int x0, int y0, int z, int y_last, float2 (*tile)[TY + 2][34]) {
     using L = Lat<DIM>;
@@ -206,10 +206,14 @@ __device__ __forceinline__ void update_tile(const StepArgs<PR>& a, const Phys<fl
     float delta = 0.f;
     if (active) {
         const unsigned mask = cross_mask<DIM>(g, x, y, z);
-        if (!fast) pull_f<DIM, PR>(a.fin, cd, g, x, y, z, self, mask, f, a.par);
+        if (!fast) pull_f<DIM, PR, kOpen>(a.fin, cd, g, x, y, z, self, mask, f, a.par);
         m = lean_moments<DIM>(f);
-        if (!fast) pull_g<DIM, PR>(a.gin, a.cin, cd, g, x, y, z, self, mask, d, cold, a.par);
-        else if (col.wraps()) unshift<DIM>(col, wc, cold, d);
+        if (!fast) {
+            pull_g<DIM, PR, kOpen>(a.gin, a.cin, cd, g, x, y, z, self, mask, d, cold, a.par);
+            if (kOpen && g.fc[0]) store_open<DIM, PR>(g, a.par, x, y, z, f, [&](int q) { return d[q]; }, cold, a.cw[self].x);
+        } else if (col.wraps()) {
+            unshift<DIM>(col, wc, cold, d);
+        }
         delta = pulled_sum<PR, Q>(d);
     }
     copy_async_wait();
@@ -231,6 +235,7 @@ __device__ __forceinline__ void update_tile(const StepArgs<PR>& a, const Phys<fl
 #pragma unroll
         for (int k = 0; k < DIM; ++k) a.u[self + unsigned(k) * unsigned(g.ps)] = u[k];
         a.cout[self] = c;
+        if (kOpen && g.fc[0]) store_open_u<DIM, PR>(g, a.par, x, y, z, a.u, self);
         if constexpr (kMon) node_monitors<DIM, PR>(a, c, u, mon);
     }
     if constexpr (kMon) store_monitor_row(a, tx, x0, y, z, mon);
@@ -242,11 +247,11 @@ __device__ __forceinline__ void update_tile(const StepArgs<PR>& a, const Phys<fl
 // registers hold it all without spills (a spilled load in flight stalls: at 80 registers and
 // 24 warps per SM the 128x256x128 update took 370 instead of 277 us).  Small blocks of 4 rows
 // keep the loads of some beside the arithmetic of others: 8 rows took 316 us, 2 rows 277.
-template <int DIM, class PR, int TY, bool kMon>
+template <int DIM, class PR, int TY, bool kOpen, bool kMon>
 __global__ void __launch_bounds__(32 * TY, 16 / TY) update_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr, int z_first) {
     __shared__ float2 tile[DIM == 3 ? 3 : 1][TY + 2][34];
     // planes in descending order: phase_kernel left the g of the highest ones in L2
-    update_tile<DIM, PR, TY, kMon>(a, a.pt, a.pp, ptr, 1 + (int)blockIdx.x * 32, 1 + (int)blockIdx.y * TY,
+    update_tile<DIM, PR, TY, kOpen, kMon>(a, a.pt, a.pp, ptr, 1 + (int)blockIdx.x * 32, 1 + (int)blockIdx.y * TY,
                                    DIM == 3 ? z_first + (int)(gridDim.z - 1 - blockIdx.z) : 0, a.g.n[1], tile);
 }
 
@@ -288,30 +293,27 @@ __global__ void __launch_bounds__(128, 8) update_batch_kernel(const StepArgs<PR>
     const BasePtrs<2, PR> ptr{a};
     const int y1 = min(by * seg + seg, a.g.n[1]);
     for (int y = by * seg + 1; y <= y1; y += 4) {
-        update_tile<2, PR, 4, false>(a, PT, PP, ptr, 1 + bx * 32, y, 0, y1, tile);
+        update_tile<2, PR, 4, false, false>(a, PT, PP, ptr, 1 + bx * 32, y, 0, y1, tile);
         __syncthreads();  // the tile is reused by the next rows
     }
 }
 
-// Rows per block and blocks per SM of update_wide_kernel.  FP64: bound by the FP64 pipe (64% busy
-// in 3D, 2,340 operations per node), the latency of its chains and instruction fetch (3,400
+// Rows per block and blocks per SM of update_fp64_kernel.  Bound by the FP64 pipe (64% busy in
+// 3D, 2,340 operations per node), the latency of its chains and instruction fetch (3,400
 // instructions in a straight line, so that warps of one block, which run close together, share
 // fetches).  3D takes 16 warps per SM as two blocks (128x256x128: 876 us per step with
 // phase_kernel; four blocks of 4 rows 900, three with 168 registers 913, five 1039; three passes
 // of one loop over the transforms 911 to 935); 2D takes 20 warps (512x2048: 117 us, with 16 125).
-template <int DIM, class PR>
-struct WideShape {
-    static constexpr int kRows = PR::kExact && DIM == 3 ? 8 : 4;
-    static constexpr int kBlocks = PR::kExact ? (DIM == 3 ? 2 : 5) : 4;
+template <int DIM>
+struct ShapeFp64 {
+    static constexpr int kRows = DIM == 3 ? 8 : 4, kBlocks = DIM == 3 ? 2 : 5;
 };
-// The same for FP64 and for cases with open sides, c read through L1.  FP64 pulls g once the new
-// velocity is known, so that its 19 values are not live through the force.
+// The FP64 update, c read through L1.  g is pulled once the new velocity is known, so that its
+// 19 values are not live through the force.
 template <int DIM, class PR, bool kOpen, bool kMon>
-__global__ void __launch_bounds__((32 * WideShape<DIM, PR>::kRows), (WideShape<DIM, PR>::kBlocks))
-    update_wide_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr) {
+__global__ void __launch_bounds__((32 * ShapeFp64<DIM>::kRows), (ShapeFp64<DIM>::kBlocks))
+    update_fp64_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr) {
     using L = Lat<DIM>;
-    using TP = typename PR::TP;
-    using T = typename PR::T;
     constexpr int Q = L::Q;
     const Geom& g = a.g;
     const Codec<PR> cd(a.pop_scale);
@@ -321,8 +323,8 @@ __global__ void __launch_bounds__((32 * WideShape<DIM, PR>::kRows), (WideShape<D
     if (x <= g.n[0] && y <= g.n[1]) {
         const unsigned self = nidx32(g, x, y, z), mask = cross_mask<DIM>(g, x, y, z);
         const Column<DIM> col(g, x, y, z);
-        const bool fast = !kOpen && !PR::kShift && !__any_sync(__activemask(), col.general);
-        T fpost[Q];
+        const bool fast = !__any_sync(__activemask(), col.general);
+        double fpost[Q];
         if (fast) {
 #pragma unroll
             for (int q = 0; q < Q; ++q) fpost[q] = cd.load_f(ptr.f_from(q, col.from(self, L::ex(q))));
@@ -331,34 +333,25 @@ __global__ void __launch_bounds__((32 * WideShape<DIM, PR>::kRows), (WideShape<D
         }
         wait_for_predecessor();
         let_successor_start();
-        const typename PR::Ring* cw = a.cw;
-        auto Cf = [&](int dx, int dy, int dz) {
+        const double* cw = a.cw;
+        auto C = [&](int dx, int dy, int dz) {
             return cw[self + unsigned(dx) + unsigned(dy) * unsigned(g.sy) + (DIM == 3 ? unsigned(dz) * unsigned(g.sz) : 0u)];
         };
-        auto Ch = [&](int dx, int dy, int dz) -> TP { return ring_hi<PR>(Cf(dx, dy, dz)); };
-        TP mu, dc[3] = {TP(0), TP(0), TP(0)};
-        phase_stencil<DIM, PR>(a.pp, Cf, mu, dc);
-        const TP cown = Ch(0, 0, 0);
-        TP gpost[Q], cold = TP(0);
-        auto gq = [&](int q) { return gpost[q]; };
+        double mu, dc[3] = {0.0, 0.0, 0.0};
+        phase_stencil<DIM, PR>(a.pp, C, mu, dc);
+        const double c = C(0, 0, 0);
+        double gpost[Q];
         auto pull = [&]() {
             if (fast) {
 #pragma unroll
                 for (int q = 0; q < Q; ++q) gpost[q] = cd.load_dev(ptr.g_from(q, col.from(self, L::ex(q))));
             } else {
+                double cold;
                 pull_g<DIM, PR, kOpen>(a.gin, a.cin, cd, g, x, y, z, self, mask, gpost, cold, a.par);
+                if (kOpen && g.fc[0]) store_open<DIM, PR>(g, a.par, x, y, z, fpost, [&](int q) { return gpost[q]; }, cold, c);
             }
-            if (kOpen && g.fc[0]) store_open<DIM, PR>(g, a.par, x, y, z, fpost, gq, cold, cown);
         };
-        if constexpr (PR::kExact) {
-            update_exact<DIM, PR>(a, cd, self, fpost, pull, gpost, cown, mu, dc, kMon ? mon : nullptr);
-        } else {
-            pull();
-            const unsigned dmask = cross_mask<DIM, true>(g, x, y, z);
-            auto cdest = [&](int q) { return dest_shift_q<DIM, PR>(q, dmask, cown, Ch); };
-            update_node<DIM, PR>(a, cd, a.pt, a.pp, self, fpost, gq, pulled_sum<PR, Q>(gpost), cold, cown, mu, dc, cdest,
-                                 kMon ? mon : nullptr);
-        }
+        update_exact<DIM, PR>(a, cd, self, fpost, pull, gpost, c, mu, dc, kMon ? mon : nullptr);
         if (kOpen && g.fc[0]) store_open_u<DIM, PR>(g, a.par, x, y, z, a.u, self);
     }
     if constexpr (kMon) store_monitor_row(a, tx, x0, y, z, mon);

@@ -278,29 +278,23 @@ struct Launch {
             ptr.fo[q] = a.fout + q * g.ps;
             ptr.go[q] = a.gout + q * g.ps;
         }
-        constexpr int TY = PR::kExact || kOpen ? WideShape<DIM, PR>::kRows : 4;
+        constexpr int TY = PR::kExact ? ShapeFp64<DIM>::kRows : 4;
         const int nx = (g.n[0] + 31) / 32, nz = DIM == 3 ? g.zhi - g.zlo + 1 : 1;
         const int py = DIM == 3 ? 8 : 4;  // rows per block of the phase field
         (void)launch_chained(phase_kernel<DIM, PR, kOpen>, dim3(nx, (g.n[1] + 2 + py - 1) / py, DIM == 3 ? nz + 2 : 1), dim3(32, py),
                              0, s, a, ptr, g.zlo - 1);
         const dim3 gu(nx, (g.n[1] + TY - 1) / TY, nz), bu(32, TY);
-        if constexpr (PR::kExact || kOpen) {
-            if constexpr (DIM == 3 && !kOpen) {
-                if (a.mon) {
-                    (void)launch_chained(update_wide_kernel<DIM, PR, kOpen, true>, gu, bu, 0, s, a, ptr);
-                    return;
-                }
-            }
-            (void)launch_chained(update_wide_kernel<DIM, PR, kOpen, false>, gu, bu, 0, s, a, ptr);
-        } else {
-            if constexpr (DIM == 3) {
-                if (a.mon) {
-                    (void)launch_chained(update_kernel<DIM, PR, TY, true>, gu, bu, 0, s, a, ptr, g.zlo);
-                    return;
-                }
-            }
-            (void)launch_chained(update_kernel<DIM, PR, TY, false>, gu, bu, 0, s, a, ptr, g.zlo);
+        auto update = [&](auto mon) {
+            constexpr bool kMon = decltype(mon)::value;
+            if constexpr (PR::kExact)
+                (void)launch_chained(update_fp64_kernel<DIM, PR, kOpen, kMon>, gu, bu, 0, s, a, ptr);
+            else
+                (void)launch_chained(update_kernel<DIM, PR, TY, kOpen, kMon>, gu, bu, 0, s, a, ptr, g.zlo);
+        };
+        if constexpr (DIM == 3 && !kOpen) {
+            if (a.mon) return update(std::true_type{});
         }
+        update(std::false_type{});
     }
 
     template <int TX, bool kKeep, bool kOpen>
