@@ -50,26 +50,55 @@ struct BasePtrs {
 };
 
 // Boundary summary of one node: element offsets that wrap a source beyond a periodic x side,
-// and whether the node needs the general pull (next to a y or z side, or to an x side that is
-// not periodic).  A quarter of the warps of a 256-wide periodic grid hold a node next to an x
-// side; these offsets cost them little, where the general pull resolves every direction of
-// every lane.
-template <int DIM>
+// whether the sources beyond its x side lie behind a wall, and whether the node needs the
+// general pull (next to a y or z side, or to an x side of another kind).  A quarter of the warps
+// of a 256-wide grid hold a node next to an x side; these cost them little, where the general
+// pull resolves every direction of every lane.
+// kWalls: the instance for cases with a wall in x (FP32/FP16; the others take the general pull
+// next to it: the choice of addresses costs a 2D step without such walls 4%, and FP64, bound by
+// its arithmetic, gains 2% with them and loses 1% without).  97x131x83 in walls 146 -> 118 us.
+template <int DIM, bool kWalls>
 struct Column {
     unsigned lo, hi;
-    bool general;
+    bool wall_lo, wall_hi, general;
     __device__ __forceinline__ Column(const Geom& g, int x, int y, int z) {
-        const bool per = g.side[0] == kSidePeriodic;
+        const bool per = g.side[0] == kSidePeriodic;  // then the other x side is as well
         lo = per && x == 1 ? unsigned(g.n[0]) : 0u;
         hi = per && x == g.n[0] ? unsigned(-g.n[0]) : 0u;
-        general = y == 1 || y == g.n[1] || (!per && (x == 1 || x == g.n[0])) || (DIM == 3 && (z == 1 || z == g.n[2]));
+        wall_lo = kWalls && x == 1 && g.side[0] == kSideWall;
+        wall_hi = kWalls && x == g.n[0] && g.side[1] == kSideWall;
+        general = y == 1 || y == g.n[1] || (!per && ((x == 1 && !wall_lo) || (x == g.n[0] && !wall_hi))) ||
+                  (DIM == 3 && (z == 1 || z == g.n[2]));
     }
     // element whose fixed lattice offset gives the source of a direction with x component ex
     __device__ __forceinline__ unsigned from(unsigned self, int ex) const {
         return ex == 0 ? self : self + (ex > 0 ? lo : hi);
     }
     __device__ __forceinline__ bool wraps() const { return (lo | hi) != 0u; }
+    __device__ __forceinline__ bool walled() const { return wall_lo || wall_hi; }
+    // a direction with x component ex bounces back at this node
+    __device__ __forceinline__ bool bounces(int ex) const { return ex > 0 ? wall_lo : (ex < 0 ? wall_hi : false); }
 };
+// The streamed populations of a node that needs no general pull: at(q, i) is the source of
+// direction q of element i (PullPtrs).  A warp without a node next to an x wall reads the fixed
+// offsets; the others choose each address between the source and the node's own opposite
+// population.
+template <int DIM, bool kWalls, typename T, class At, class Load>
+__device__ __forceinline__ void pull_column(const Geom& g, const Column<DIM, kWalls>& col, unsigned self, T* v, At at, Load load) {
+    using L = Lat<DIM>;
+    if (kWalls && __any_sync(__activemask(), col.walled())) {
+#pragma unroll
+        for (int q = 0; q < L::Q; ++q) {
+            const int o = opposite<DIM>(q);
+            auto* src = at(q, col.from(self, L::ex(q)));
+            auto* own = at(o, self - pull_offset<DIM>(g, o) + unsigned(o) * unsigned(g.ps));
+            v[q] = load(col.bounces(L::ex(q)) ? own : src);
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < L::Q; ++q) v[q] = load(at(q, col.from(self, L::ex(q))));
+    }
+}
 
 // Shifted storage: the g that crossed a periodic x side were stored shifted by their own node's
 // c (see Prec).  wrapped_c requests the c of those sources, unshift brings the values to this
@@ -84,8 +113,8 @@ __host__ __device__ constexpr int from_high(int i) {
         if (Lat<DIM>::ex(m) == -1 && Lat<DIM>::ey(m) == Lat<DIM>::ey(q) && Lat<DIM>::ez(m) == Lat<DIM>::ez(q)) return m;
     return 0;
 }
-template <int DIM, class A>
-__device__ __forceinline__ void wrapped_c(const A* __restrict__ C, const Geom& g, const Column<DIM>& col, unsigned self,
+template <int DIM, bool kWalls, class A>
+__device__ __forceinline__ void wrapped_c(const A* __restrict__ C, const Geom& g, const Column<DIM, kWalls>& col, unsigned self,
                                           A* wc) {
     const unsigned s = self + col.lo + col.hi + (col.lo ? 0u : 2u);
 #pragma unroll
@@ -94,8 +123,8 @@ __device__ __forceinline__ void wrapped_c(const A* __restrict__ C, const Geom& g
         wc[i] = C[s + pull_offset<DIM>(g, q) - unsigned(q) * unsigned(g.ps)];
     }
 }
-template <int DIM>
-__device__ __forceinline__ void unshift(const Column<DIM>& col, const float* wc, float cself, float* v) {
+template <int DIM, bool kWalls>
+__device__ __forceinline__ void unshift(const Column<DIM, kWalls>& col, const float* wc, float cself, float* v) {
 #pragma unroll
     for (int i = 0; i < Lat<DIM>::A; ++i) {
         const int up = from_low<DIM>(i), dn = from_high<DIM>(i);
@@ -110,7 +139,7 @@ __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcon
 
 // c of this step at (x, y, z), ghost coordinates included (x an interior node's: its neighbours
 // in the x ghost columns with it).
-template <int DIM, class PR, bool kOpen, class Ptr>
+template <int DIM, class PR, bool kOpen, bool kWalls, class Ptr>
 __device__ __forceinline__ void phase_node(const StepArgs<PR>& a, const Ptr& ptr, int x, int y, int z) {
     using L = Lat<DIM>;
     using TP = typename PR::TP;
@@ -120,19 +149,18 @@ __device__ __forceinline__ void phase_node(const StepArgs<PR>& a, const Ptr& ptr
     const unsigned self = nidx32(g, x, y, z);
     typename PR::Ring c;
     if (y >= 1 && y <= g.n[1] && (DIM == 2 || (z >= 1 && z <= g.n[2]))) {
-        const Column<DIM> col(g, x, y, z);
+        const Column<DIM, kWalls> col(g, x, y, z);
         TP v[L::Q], cs = TP(0);
         if (__any_sync(__activemask(), col.general)) {
             pull_g<DIM, PR, kOpen>(a.gin, a.cin, cd, g, x, y, z, self, cross_mask<DIM>(g, x, y, z), v, cs, a.par);
         } else {
             if constexpr (PR::kShift) cs = a.cin[self];
-#pragma unroll
-            for (int q = 0; q < L::Q; ++q) v[q] = cd.load_dev(ptr.g_from(q, col.from(self, L::ex(q))));
+            pull_column(g, col, self, v, [&](int q, unsigned i) { return ptr.g_from(q, i); }, [&](auto* p) { return cd.load_dev(p); });
             if constexpr (PR::kShift)
                 if (col.wraps()) {
                     float wc[L::A];
-                    wrapped_c<DIM>(a.cin, g, col, self, wc);
-                    unshift<DIM>(col, wc, cs, v);
+                    wrapped_c(a.cin, g, col, self, wc);
+                    unshift(col, wc, cs, v);
                 }
         }
         c = ring_c<PR>(pulled_sum<PR, L::Q>(v), cs);
@@ -147,13 +175,13 @@ __device__ __forceinline__ void phase_node(const StepArgs<PR>& a, const Ptr& ptr
 // Bound by memory: 70 us on the 128x256x128 bubble in FP32, 88 bytes per node at 5.3 TB/s (79
 // us, 382 instead of 230 instructions per node, with the general pull in every warp next to a
 // side).
-template <int DIM, class PR, bool kOpen>
+template <int DIM, class PR, bool kOpen, bool kWalls>
 __global__ void __launch_bounds__(256) phase_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr, int z_first) {
     const int x = 1 + (int)(blockIdx.x * 32 + threadIdx.x), y = (int)(blockIdx.y * blockDim.y + threadIdx.y);
     // in this order: the update may start once everything before this kernel has ended
     wait_for_predecessor();
     let_successor_start();
-    if (x <= a.g.n[0] && y <= a.g.n[1] + 1) phase_node<DIM, PR, kOpen>(a, ptr, x, y, DIM == 3 ? z_first + (int)blockIdx.z : 0);
+    if (x <= a.g.n[0] && y <= a.g.n[1] + 1) phase_node<DIM, PR, kOpen, kWalls>(a, ptr, x, y, DIM == 3 ? z_first + (int)blockIdx.z : 0);
 }
 
 // 8 bytes from global to shared memory without a register between (completion: copy_async_wait
@@ -165,7 +193,7 @@ __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_
 
 // FP32/FP16 update of the 32 x TY tile of a plane whose first node is (x0, y0, z), rows up to
 // y_last, one node per thread.  PT: a.pt, PP: a.pp (or copies of them in registers).
-template <int DIM, class PR, int TY, bool kOpen, bool kMon, class Ptr>
+template <int DIM, class PR, int TY, bool kOpen, bool kWalls, bool kMon, class Ptr>
 __device__ __forceinline__ void update_tile(const StepArgs<PR>& a, const Phys<float>& PT, const Phys<float>& PP, const Ptr& ptr,
                                             int x0, int y0, int z, int y_last, float2 (*tile)[TY + 2][34]) {
     using L = Lat<DIM>;
@@ -175,16 +203,14 @@ __device__ __forceinline__ void update_tile(const StepArgs<PR>& a, const Phys<fl
     const int tx = threadIdx.x, ty = threadIdx.y, x = x0 + tx, y = y0 + ty;
     const bool active = x <= g.n[0] && y <= y_last;
     const unsigned self = nidx32(g, x, y, z);
-    const Column<DIM> col(g, x, y, z);
+    const Column<DIM, kWalls> col(g, x, y, z);
     const bool fast = !__any_sync(0xffffffffu, active && col.general);
     float f[Q], d[Q], u[3], cold = 0.f, wc[L::A];
     if (active) {
         if (fast) {
-#pragma unroll
-            for (int q = 0; q < Q; ++q) f[q] = cd.load_f(ptr.f_from(q, col.from(self, L::ex(q))));
-#pragma unroll
-            for (int q = 0; q < Q; ++q) d[q] = cd.load_dev(ptr.g_from(q, col.from(self, L::ex(q))));
-            if (col.wraps()) wrapped_c<DIM>(a.cin, g, col, self, wc);
+            pull_column(g, col, self, f, [&](int q, unsigned i) { return ptr.f_from(q, i); }, [&](auto* p) { return cd.load_f(p); });
+            pull_column(g, col, self, d, [&](int q, unsigned i) { return ptr.g_from(q, i); }, [&](auto* p) { return cd.load_dev(p); });
+            if (col.wraps()) wrapped_c(a.cin, g, col, self, wc);
         }
         cold = a.cin[self];
 #pragma unroll
@@ -212,7 +238,7 @@ __device__ __forceinline__ void update_tile(const StepArgs<PR>& a, const Phys<fl
             pull_g<DIM, PR, kOpen>(a.gin, a.cin, cd, g, x, y, z, self, mask, d, cold, a.par);
             if (kOpen && g.fc[0]) store_open<DIM, PR>(g, a.par, x, y, z, f, [&](int q) { return d[q]; }, cold, a.cw[self].x);
         } else if (col.wraps()) {
-            unshift<DIM>(col, wc, cold, d);
+            unshift(col, wc, cold, d);
         }
         delta = pulled_sum<PR, Q>(d);
     }
@@ -247,11 +273,11 @@ __device__ __forceinline__ void update_tile(const StepArgs<PR>& a, const Phys<fl
 // registers hold it all without spills (a spilled load in flight stalls: at 80 registers and
 // 24 warps per SM the 128x256x128 update took 370 instead of 277 us).  Small blocks of 4 rows
 // keep the loads of some beside the arithmetic of others: 8 rows took 316 us, 2 rows 277.
-template <int DIM, class PR, int TY, bool kOpen, bool kMon>
+template <int DIM, class PR, int TY, bool kOpen, bool kWalls, bool kMon>
 __global__ void __launch_bounds__(32 * TY, 16 / TY) update_kernel(StepArgs<PR> a, PullPtrs<DIM, PR> ptr, int z_first) {
     __shared__ float2 tile[DIM == 3 ? 3 : 1][TY + 2][34];
     // planes in descending order: phase_kernel left the g of the highest ones in L2
-    update_tile<DIM, PR, TY, kOpen, kMon>(a, a.pt, a.pp, ptr, 1 + (int)blockIdx.x * 32, 1 + (int)blockIdx.y * TY,
+    update_tile<DIM, PR, TY, kOpen, kWalls, kMon>(a, a.pt, a.pp, ptr, 1 + (int)blockIdx.x * 32, 1 + (int)blockIdx.y * TY,
                                    DIM == 3 ? z_first + (int)(gridDim.z - 1 - blockIdx.z) : 0, a.g.n[1], tile);
 }
 
@@ -279,7 +305,7 @@ __global__ void __launch_bounds__(128) phase_batch_kernel(const StepArgs<PR>* __
     if (x > a.g.n[0]) return;
     const BasePtrs<2, PR> ptr{a};
     for (int y = (by == 0 ? 0 : by * seg + 1) + (int)threadIdx.y; y <= (last == n1 ? n1 + 1 : last); y += 4)
-        phase_node<2, PR, false>(a, ptr, x, y, 0);
+        phase_node<2, PR, false, false>(a, ptr, x, y, 0);
 }
 template <class PR>
 __global__ void __launch_bounds__(128, 8) update_batch_kernel(const StepArgs<PR>* __restrict__ args, const int* __restrict__ items, int seg) {
@@ -293,7 +319,7 @@ __global__ void __launch_bounds__(128, 8) update_batch_kernel(const StepArgs<PR>
     const BasePtrs<2, PR> ptr{a};
     const int y1 = min(by * seg + seg, a.g.n[1]);
     for (int y = by * seg + 1; y <= y1; y += 4) {
-        update_tile<2, PR, 4, false, false>(a, PT, PP, ptr, 1 + bx * 32, y, 0, y1, tile);
+        update_tile<2, PR, 4, false, false, false>(a, PT, PP, ptr, 1 + bx * 32, y, 0, y1, tile);
         __syncthreads();  // the tile is reused by the next rows
     }
 }
@@ -322,12 +348,11 @@ __global__ void __launch_bounds__((32 * ShapeFp64<DIM>::kRows), (ShapeFp64<DIM>:
     double mon[2] = {0.0, 0.0};
     if (x <= g.n[0] && y <= g.n[1]) {
         const unsigned self = nidx32(g, x, y, z), mask = cross_mask<DIM>(g, x, y, z);
-        const Column<DIM> col(g, x, y, z);
+        const Column<DIM, false> col(g, x, y, z);
         const bool fast = !__any_sync(__activemask(), col.general);
         double fpost[Q];
         if (fast) {
-#pragma unroll
-            for (int q = 0; q < Q; ++q) fpost[q] = cd.load_f(ptr.f_from(q, col.from(self, L::ex(q))));
+            pull_column(g, col, self, fpost, [&](int q, unsigned i) { return ptr.f_from(q, i); }, [&](auto* p) { return cd.load_f(p); });
         } else {
             pull_f<DIM, PR, kOpen>(a.fin, cd, g, x, y, z, self, mask, fpost, a.par);
         }
@@ -343,8 +368,7 @@ __global__ void __launch_bounds__((32 * ShapeFp64<DIM>::kRows), (ShapeFp64<DIM>:
         double gpost[Q];
         auto pull = [&]() {
             if (fast) {
-#pragma unroll
-                for (int q = 0; q < Q; ++q) gpost[q] = cd.load_dev(ptr.g_from(q, col.from(self, L::ex(q))));
+                pull_column(g, col, self, gpost, [&](int q, unsigned i) { return ptr.g_from(q, i); }, [&](auto* p) { return cd.load_dev(p); });
             } else {
                 double cold;
                 pull_g<DIM, PR, kOpen>(a.gin, a.cin, cd, g, x, y, z, self, mask, gpost, cold, a.par);

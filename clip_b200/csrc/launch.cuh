@@ -268,6 +268,12 @@ struct Launch {
     // The two-pass step (kernels_split.cuh).
     template <int DIM, bool kOpen>
     static void go_split(const DevState& st, const StepArgs<PR>& a, cudaStream_t s) {
+        if constexpr (!PR::kExact && !kOpen)
+            if (st.g.side[0] == kSideWall || st.g.side[1] == kSideWall) return go_split_on<DIM, kOpen, true>(st, a, s);
+        go_split_on<DIM, kOpen, false>(st, a, s);
+    }
+    template <int DIM, bool kOpen, bool kWalls>
+    static void go_split_on(const DevState& st, const StepArgs<PR>& a, cudaStream_t s) {
         using L = Lat<DIM>;
         const Geom& g = st.g;
         PullPtrs<DIM, PR> ptr;
@@ -281,7 +287,7 @@ struct Launch {
         constexpr int TY = PR::kExact ? ShapeFp64<DIM>::kRows : 4;
         const int nx = (g.n[0] + 31) / 32, nz = DIM == 3 ? g.zhi - g.zlo + 1 : 1;
         const int py = DIM == 3 ? 8 : 4;  // rows per block of the phase field
-        (void)launch_chained(phase_kernel<DIM, PR, kOpen>, dim3(nx, (g.n[1] + 2 + py - 1) / py, DIM == 3 ? nz + 2 : 1), dim3(32, py),
+        (void)launch_chained(phase_kernel<DIM, PR, kOpen, kWalls>, dim3(nx, (g.n[1] + 2 + py - 1) / py, DIM == 3 ? nz + 2 : 1), dim3(32, py),
                              0, s, a, ptr, g.zlo - 1);
         const dim3 gu(nx, (g.n[1] + TY - 1) / TY, nz), bu(32, TY);
         auto update = [&](auto mon) {
@@ -289,7 +295,7 @@ struct Launch {
             if constexpr (PR::kExact)
                 (void)launch_chained(update_fp64_kernel<DIM, PR, kOpen, kMon>, gu, bu, 0, s, a, ptr);
             else
-                (void)launch_chained(update_kernel<DIM, PR, TY, kOpen, kMon>, gu, bu, 0, s, a, ptr, g.zlo);
+                (void)launch_chained(update_kernel<DIM, PR, TY, kOpen, kWalls, kMon>, gu, bu, 0, s, a, ptr, g.zlo);
         };
         if constexpr (DIM == 3 && !kOpen) {
             if (a.mon) return update(std::true_type{});
