@@ -60,6 +60,15 @@ struct clipb_batch {
 
 namespace {
 
+// Whether every case can run the variant (the FP32/FP16 two-pass step needs its work arrays).
+bool launchable(const clipb_batch* b, int variant) {
+    for (const auto* c : b->cases) {
+        if (!b->kt.available(c->st, variant)) return false;
+        if (b->precision != CLIPB_FP64 && variant == b->kt.default_variant(c->st) && !c->st.cw) return false;
+    }
+    return true;
+}
+
 // Work items (case, tile bx, row segment by) for a tile width and segment length, case by
 // case so that CTAs running at the same time work on neighbouring tiles of one case.
 int build_items(clipb_batch* b) {
@@ -184,7 +193,8 @@ int clipb_batch_create(const char* const* configs, int ncases, int kind, int pre
         s->stream = b->stream;  // every case runs on the batch's stream
     }
     b->kt = b->cases[0]->kt;
-    if (precision != CLIPB_FP64) {  // the two-pass step (its rates: update_batch_kernel)
+    if (precision != CLIPB_FP64 && launchable(b.get(), b->kt.default_variant(b->cases[0]->st))) {
+        // the two-pass step (its rates: update_batch_kernel)
         b->variant = b->kt.default_variant(b->cases[0]->st);
         b->seg = 16;
     }
@@ -269,7 +279,7 @@ int clipb_batch_solve_sequential(clipb_batch* b, int nsteps) {
 
 int clipb_batch_set_launch(clipb_batch* b, int variant, int seg, int blocks_per_sm) {
     if (!b) return fail(CLIPB_E_ARG, "null batch");
-    if (variant < 0 || variant >= b->kt.variants2 || !b->kt.available(b->cases[0]->st, variant))
+    if (variant < 0 || variant >= b->kt.variants2 || !launchable(b, variant))
         return fail(CLIPB_E_ARG, "variant must be in [0, " + std::to_string(b->kt.variants2) + ")");
     if (seg < 1) return fail(CLIPB_E_ARG, "rows per work item must be positive");
     if (blocks_per_sm < 0) return fail(CLIPB_E_ARG, "negative blocks per SM");
@@ -325,7 +335,7 @@ int clipb_batch_autotune(clipb_batch* b, int trial_steps, int* best_variant, int
     float best = 1e30f;
     int bv = b->variant, bs = b->seg, bb = b->blocks_per_sm, rc;
     for (int v = 0; v < b->kt.variants2; ++v) {
-        if (!b->kt.available(b->cases[0]->st, v)) continue;
+        if (!launchable(b, v)) continue;
         for (int seg : {4, 8, 16, 32, 64})
             for (int bps : {1, 2, 0}) {
                 if (bps && b->precision != CLIPB_FP64 && !b->kt.marches(b->cases[0]->st, v)) continue;  // not persistent

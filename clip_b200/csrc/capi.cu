@@ -180,12 +180,16 @@ int clipb::solver_create(const CaseConfig& cfg, int precision, clipb_solver** ou
         }
     }
     if ((rc = s->alloc(&st.p, aux))) return rc;
-    if ((rc = s->alloc(&st.cw, (size_t)g.ps * 8))) return rc;
     if ((rc = s->alloc((void**)&st.c0, (size_t)g.ps * sizeof(double)))) return rc;
     st.red_blocks = 8 * 148;  // monitor blocks: a fixed count keeps the sums deterministic
     if ((rc = s->alloc((void**)&st.red, (size_t)2 * st.red_blocks * sizeof(double)))) return rc;
     if ((rc = s->alloc((void**)&s->d_mon, 3 * sizeof(double)))) return rc;
     if ((rc = s->alloc((void**)&st.err, sizeof(int)))) return rc;
+    // the two-pass step's work array comes last: where it does not fit, the step marches instead
+    if (s->alloc(&st.cw, (size_t)g.ps * 8)) {
+        st.cw = nullptr;
+        (void)cudaGetLastError();
+    }
     CLIPB_CUDA(cudaMallocHost((void**)&s->h_mon, 4 * sizeof(double)));  // the last one: the wait flag
     // staged variants need tensor maps of the buffers; without them they are unavailable
     if (s->kt.prepare(st) != cudaSuccess) {

@@ -99,7 +99,7 @@ struct DevState {
     // monitor partials written by a monitored 3D step (mass and kinetic energy of each row
     // segment of 32 nodes, 2 doubles each), or null: set only for that step's launch
     double* mon_rows;
-    void* cw;            // two-pass step: c of the step (8 bytes per node)
+    void* cw;            // two-pass step: c of the step (8 bytes per node); null: no memory for it
     double pop_scale;    // FP16: power-of-two scale of stored f
     int variant;         // launch variant of the fused step (Launch::step)
     int seg;             // planes (3D) / rows (2D) per CTA; 0 = default

@@ -325,8 +325,10 @@ struct Launch {
     // kOpen: the kernel instances for cases with free-convect or Neumann sides.
     template <bool kOpen>
     static void step_shape(const DevState& st, const StepArgs<PR>& a, long long k, cudaStream_t s) {
+        // without its work array the two-pass step's variant is the march of variant 0
+        const int variant = !st.cw && st.variant == default_variant(st) ? 0 : st.variant;
         if (st.g.dim == 3) {
-            switch (st.variant) {
+            switch (variant) {
                 case 1: go3<32, 8, kKeepG3, kOpen>(st, a, s); break;
                 case 2: go3<32, 16, false, kOpen>(st, a, s); break;
                 case 3: go3<64, 8, false, kOpen>(st, a, s); break;
@@ -350,7 +352,7 @@ struct Launch {
                 default: go3<32, 8, false, kOpen>(st, a, s); break;
             }
         } else {
-            switch (st.variant) {
+            switch (variant) {
                 case 1: go2<32, kKeepG2, kOpen>(st, a, s); break;
                 case 2: go2<128, kKeepG2, kOpen>(st, a, s); break;
                 case 3: go_split<2, kOpen>(st, a, s); break;

@@ -169,8 +169,8 @@ int clipb_get_field_device(clipb_solver* s, int field, double* dev_out, size_t c
 int clipb_monitors(clipb_solver* s, double* mass, double* kinetic);
 
 /* nsteps steps (>= 1) and the monitors of the state they leave, as clipb_solve followed by
- * clipb_monitors, with the reduction folded into the last step: on the 3D direct-load
- * launch variants that step sums the mass and kinetic energy of each row segment of 32
+ * clipb_monitors, with the reduction folded into the last step: on the 3D two-pass
+ * and direct-load launch variants that step sums the mass and kinetic energy of each row segment of 32
  * nodes as it stores c and u, and two short passes add those partials in a fixed order, so
  * the stored state is not read again.  The result does not depend on the launch variant or
  * the planes per CTA; it differs from clipb_monitors' only by the order of the FP64
@@ -182,9 +182,13 @@ int clipb_solve_monitored(clipb_solver* s, int nsteps, double* mass, double* kin
  * elapsed device time.  No reference counterpart (the reference has no timers). */
 int clipb_time_steps(clipb_solver* s, int nsteps, float* ms);
 
-/* Launch shape of the fused step: `variant` selects a tile shape / register policy
- * (0 .. nvariants-1), `seg` the planes (3D) or rows (2D) each thread block marches over
- * (0 = default: 2D takes the longest of 16, 8, 4, 2 rows that leaves eight blocks per SM).  Results do not depend on the launch shape.  No reference counterpart
+/* Launch shape of the step: `variant` selects the two-pass step or a tile shape / register
+ * policy of the marching one (0 .. nvariants-1), `seg` the planes (3D) or rows (2D) each
+ * thread block marches over (0 = default: 2D takes the longest of 16, 8, 4, 2 rows that
+ * leaves eight blocks per SM).  The two-pass step (variant 7 in 3D FP32/FP16, 4 in 3D FP64,
+ * 3 in 2D; a new solver's default) ignores seg; it keeps c of the step in 8 more bytes per
+ * node, and a solver created without room for them marches with variant 0 instead.  Results
+ * do not depend on the launch shape.  No reference counterpart
  * (the reference launches fixed 8x8(x4) blocks, DataArray.cu:27-44). */
 int clipb_set_launch(clipb_solver* s, int variant, int seg);
 int clipb_get_launch(const clipb_solver* s, int* variant, int* seg, int* nvariants);
@@ -386,7 +390,9 @@ int clipb_batch_solve(clipb_batch* b, int nsteps);
 int clipb_batch_solve_sequential(clipb_batch* b, int nsteps);
 
 /* Launch shape of the batched step: 2D tile variant (as clipb_set_launch), rows per work
- * item, persistent thread blocks per SM (0: as many as fit).  Results do not depend on it. */
+ * item, persistent thread blocks per SM (0: as many as fit).  FP32/FP16 variant 3, the
+ * default there, is the two-pass step: one block per work item, blocks_per_sm unused.
+ * Results do not depend on it. */
 int clipb_batch_set_launch(clipb_batch* b, int variant, int rows_per_item, int blocks_per_sm);
 int clipb_batch_get_launch(const clipb_batch* b, int* variant, int* rows_per_item, int* blocks_per_sm, int* nitems);
 

@@ -85,3 +85,32 @@ def test_two_pass_batch_equals_the_march(prec, rows):
             out.append([b.case(i).interior_field(f) for i in range(5) for f in ("c", "vel", "g")])
     for a, b in zip(*out):
         assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_two_pass_work_array_is_optional(tmp_path, prec):
+    """A solver whose state fits but not the work array is created all the same, and marches."""
+    import torch
+
+    path = _config(tmp_path / "config.txt", (8192, 1024), "pw")
+    with cb.Solver(path, prec) as s:
+        need = s.info().device_bytes
+        s.set_launch(0, 0)
+        s.init()
+        s.solve(3)
+        want = s.interior_field("f_post")
+        s.set_launch(3, 0)  # loads its kernels too
+        s.solve(1)
+    work = 8192 * 1024 * 8  # at least; allocations round up to 2 MB
+    torch.cuda.empty_cache()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - (need - work // 4), dtype=torch.uint8, device="cuda")
+    s = cb.Solver(path, prec)
+    del filler
+    torch.cuda.empty_cache()
+    try:
+        assert s.info().device_bytes <= need - work
+        s.init()
+        s.solve(3)
+        assert np.array_equal(s.interior_field("f_post"), want)
+    finally:
+        s.close()
