@@ -4,7 +4,8 @@
 Workload: 3D rising bubble, D3Q19 + D3Q19 phase field, 256x512x256 interior nodes
 (clip_b200/workloads/bubble3d_256x512x256.txt; the vertical axis is y as in the
 reference's config semantics), synthetic initial state from the config (no dataset).
-A step is one time step of the whole grid: one fused kernel launch.
+A step is one time step of the whole grid: two kernel launches (the phase
+field, then the update) or, on the marching launch variants, one.
 
 Our arm (default): FP32 population storage (the production precision); FP64 and FP16
 storage are timed on the same workload and reported as extra keys.  The timed region
@@ -37,6 +38,7 @@ sys.path.insert(0, REPO)
 WORKLOAD = os.path.join(REPO, "clip_b200", "workloads", "bubble3d_256x512x256.txt")
 WORKLOAD_NAME = "3d_rising_bubble_256x512x256"
 METRIC = "MLUPS"
+TWO_PASS = 7  # launch variant of the 3D FP32/FP16 two-pass step (two kernels per step)
 # Algorithmic bytes per lattice update: f and g read + written once (2 * 2Q values) and
 # u, c read + written once (2 * (DIM + 1) values).
 Q, DIM = 19, 3
@@ -55,7 +57,7 @@ def _peaks():
 
 
 def _profile_traffic(dtype):
-    """DRAM bytes per lattice update of the fused kernel from the committed ncu summary."""
+    """DRAM bytes per lattice update of the step's kernels from the committed ncu summary."""
     try:
         with open(os.path.join(REPO, "profiles", "ncu_traffic.json")) as fp:
             d = json.load(fp)
@@ -336,7 +338,8 @@ def run_ours(args, world, rank, local):
     if rank == 0 and args.err_steps > 0:
         results["precision_vs_fp64"] = precision_errors(args.err_steps, args.err_block)
     barrier(world)
-    launches = args.steps  # one fused kernel per step, no inlet on this workload
+    # no inlet on this workload: the marching variants are one kernel per step, the two-pass one two
+    launches = args.steps * (2 if results["launch"]["fp32"]["variant"] == TWO_PASS else 1)
     return results, launches
 
 
@@ -349,7 +352,6 @@ def run_slabs(k=4, steps=20, check_steps=10, ms_whole=None):
     from clip_b200.slabs import SlabGroup
 
     whole = cb.Solver(WORKLOAD, "fp32")
-    whole.set_launch(8, 8)
     whole.init()
     whole.set_graphs(False)
     whole.solve(check_steps)
@@ -357,7 +359,7 @@ def run_slabs(k=4, steps=20, check_steps=10, ms_whole=None):
     whole.close()
     out = {}
     for overlap in (False, True):
-        with SlabGroup(WORKLOAD, "fp32", k, variant=8, seg=8, overlap=overlap) as grp:
+        with SlabGroup(WORKLOAD, "fp32", k, overlap=overlap) as grp:
             grp.init()
             grp.solve(check_steps)
             exact = bool(np.array_equal(grp.field("c"), c_whole))
@@ -374,8 +376,8 @@ def run_slabs(k=4, steps=20, check_steps=10, ms_whole=None):
             "ms_per_step_overlap": out["overlap"][0], "ms_per_step_whole": ms_whole,
             "exchange_bytes_per_step": 2 * 2 * k * packet,
             "bit_exact_vs_whole_after_steps": check_steps if out["serial"][1] and out["overlap"][1] else None,
-            "timed": f"{steps} steps of k slabs on one GPU, CUDA events on the slabs' stream: serial = k fused "
-                     "steps then 2k pack and 2k unpack launches; overlap = the face planes of each slab first, "
+            "timed": f"{steps} steps of k slabs on one GPU, CUDA events on the slabs' stream: serial = k "
+                     "steps (two kernels each) then 2k pack and 2k unpack launches; overlap = the face planes of each slab first, "
                      "then the packs and unpacks on a second stream while the other planes update"}
 
 
@@ -391,7 +393,7 @@ def run_slab_ranks(args, world, rank, local):
     torch.cuda.set_device(local)
     dist.init_process_group("nccl", timeout=timedelta(seconds=120))
     interior = 256 * 512 * 256
-    ds = DistributedSlab(WORKLOAD, "fp32", variant=8, seg=8, overlap=True)
+    ds = DistributedSlab(WORKLOAD, "fp32", overlap=True)
     ds.init()
     ds.solve(args.warmup)
     torch.cuda.synchronize()
@@ -406,10 +408,11 @@ def run_slab_ranks(args, world, rank, local):
     barrier(world)
     sampler.__exit__(None, None, None)
     ms = max_over_ranks(e0.elapsed_time(e1), world)
-    # per step and rank: the two parts of the step, one pack per send and one unpack per receive
+    # per step and rank: the step's two kernels over the planes next to each face and over the
+    # rest (three ranges of planes), one pack per send and one unpack per receive
     sends = sum(1 for phase in ds._plan for op in phase if op[0] == "send")
     recvs = sum(1 for phase in ds._plan for op in phase if op[0] == "recv")
-    launches = args.steps * (2 + sends + recvs)
+    launches = args.steps * (3 * 2 + sends + recvs)
     nodes_rank = 256 * 512 * (ds.slab.zhi - ds.slab.zlo + 1)
     peak, peak_kind = _peaks()
     per_rank_gbs = B_LU["f32"] * nodes_rank * args.steps / (ms * 1e-3) / 1e9
