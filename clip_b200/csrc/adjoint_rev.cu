@@ -172,12 +172,13 @@ __device__ __forceinline__ void force_rev(const double* uu, const Force& o, doub
 }
 
 // Block shape of the node kernel, and the operands each thread stages in shared memory
-// before it computes: the adjoints of its 9 f and 9 g outputs (taken where the next step
-// pulls them), its 9 pulled f and 9 pulled g, and c over its 3 x 3 neighbourhood.  Staging
-// issues these 45 scattered loads together; nodes one away from every side (whole warps,
-// mostly) find them at fixed offsets.
+// before it computes: the adjoints of its 9 f and 9 g outputs and of the c their g were summed
+// into (taken where the next step pulls them), its 9 pulled f and 9 pulled g, and c over its
+// 3 x 3 neighbourhood.  These 54 scattered operands arrive by asynchronous copies, all in flight
+// without a register each; nodes one away from every side (whole warps, mostly) find them at
+// fixed offsets.  108 KB per block, two blocks per SM.
 constexpr int kNodeThreads = 256;
-constexpr int kSlf = 0, kSlg = Q, kSgp = 2 * Q, kSfp = 3 * Q, kSc = 4 * Q, kStage = 4 * Q + 9;
+constexpr int kSlf = 0, kSlg = Q, kSgp = 2 * Q, kSfp = 3 * Q, kSc = 4 * Q, kSlc = kSc + 9, kStage = kSlc + Q;
 constexpr int kNodeSmem = kStage * kNodeThreads * (int)sizeof(double);
 
 // acc += k v for a lattice factor k in {-1, 0, 1}, known once the direction loops are
@@ -187,12 +188,17 @@ __device__ __forceinline__ void acc_k(double& acc, int k, double v) {
     else if (k < 0) acc -= v;
 }
 
-// Stage the node's operands into its column st[row * kNodeThreads] of the stage.
-__device__ __forceinline__ void stage_node(const Geom& g, int x, int y, const Tape& in, const double* c_out,
-                                           const AdjBufs& A, int par, double* st) {
+// Asynchronous copy of one operand into the thread's own column of the stage; staged() waits
+// for the thread's copies.
+__device__ __forceinline__ void stage8(double* to, const double* from) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+}
+__device__ __forceinline__ void staged() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Stage the node's operands into its column st[row * kNodeThreads] of the stage: those of
+// the tape (the pulled populations and the c neighbourhood) ...
+__device__ __forceinline__ void stage_tape(const Geom& g, int x, int y, const Tape& in, const double* c_out, double* st) {
     constexpr int NT = kNodeThreads;
-    const double* lfp_in = par ? A.lfp[0] : A.lfp[1];
-    const double* lgp_in = par ? A.lgp[0] : A.lgp[1];
     const long long self = nidx(g, x, y, 0), ps = g.ps;
     if (x > 1 && x < g.n[0] && y > 1 && y < g.n[1]) {
         // every neighbour is interior: fixed 32-bit offsets (Q planes hold fewer than 2^32
@@ -200,36 +206,55 @@ __device__ __forceinline__ void stage_node(const Geom& g, int x, int y, const Ta
         const unsigned s32 = (unsigned)self, p32 = (unsigned)ps, sy = (unsigned)g.sy;
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
-            const unsigned off = unsigned(L2::ex(q)) + unsigned(L2::ey(q)) * sy;
-            const unsigned d = s32 + off, s = s32 - off, qo = unsigned(q) * p32;
-            st[(kSlf + q) * NT] = lfp_in[qo + d];
-            st[(kSlg + q) * NT] = lgp_in[qo + d] + A.lcf[d];
-            st[(kSgp + q) * NT] = in.g[qo + s];
-            st[(kSfp + q) * NT] = in.f[qo + s];
+            const unsigned s = s32 - unsigned(L2::ex(q)) - unsigned(L2::ey(q)) * sy, qo = unsigned(q) * p32;
+            stage8(st + (kSgp + q) * NT, in.g + (qo + s));
+            stage8(st + (kSfp + q) * NT, in.f + (qo + s));
         }
 #pragma unroll
         for (int oy = -1; oy <= 1; ++oy)
 #pragma unroll
             for (int ox = -1; ox <= 1; ++ox)
-                st[(kSc + 3 * (oy + 1) + ox + 1) * NT] = c_out[s32 + unsigned(ox) + unsigned(oy) * sy];
+                stage8(st + (kSc + 3 * (oy + 1) + ox + 1) * NT, c_out + (s32 + unsigned(ox) + unsigned(oy) * sy));
     } else {
         for (int q = 0; q < Q; ++q) {
-            int qd, qs;
+            int qs;
             bool crossed;
-            const long long d = stream_dest(g, x, y, q, qd);
             const long long s = pull_source<2>(g, q, x, y, 0, self, qs, crossed);
-            st[(kSlf + q) * NT] = lfp_in[qd * ps + d];
-            st[(kSlg + q) * NT] = lgp_in[qd * ps + d] + A.lcf[d];
-            st[(kSgp + q) * NT] = in.g[qs * ps + s];
-            st[(kSfp + q) * NT] = in.f[qs * ps + s];
+            stage8(st + (kSgp + q) * NT, in.g + qs * ps + s);
+            stage8(st + (kSfp + q) * NT, in.f + qs * ps + s);
         }
         // interior: this step's c; ghosts: the lagged c of step k
         for (int oy = -1; oy <= 1; ++oy)
             for (int ox = -1; ox <= 1; ++ox) {
                 const int xx = x + ox, yy = y + oy;
-                st[(kSc + 3 * (oy + 1) + ox + 1) * NT] =
-                    interior2(g, xx, yy) ? c_out[nidx(g, xx, yy, 0)] : in.c[ghost_source(g, xx, yy)];
+                stage8(st + (kSc + 3 * (oy + 1) + ox + 1) * NT,
+                       interior2(g, xx, yy) ? c_out + nidx(g, xx, yy, 0) : in.c + ghost_source(g, xx, yy));
             }
+    }
+}
+// ... and the adjoints of its outputs, which the previous kernels of the sweep write.
+__device__ __forceinline__ void stage_adjoints(const Geom& g, int x, int y, const AdjBufs& A, int par, double* st) {
+    constexpr int NT = kNodeThreads;
+    const double* lfp_in = par ? A.lfp[0] : A.lfp[1];
+    const double* lgp_in = par ? A.lgp[0] : A.lgp[1];
+    const long long self = nidx(g, x, y, 0), ps = g.ps;
+    if (x > 1 && x < g.n[0] && y > 1 && y < g.n[1]) {
+        const unsigned s32 = (unsigned)self, p32 = (unsigned)ps, sy = (unsigned)g.sy;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const unsigned d = s32 + unsigned(L2::ex(q)) + unsigned(L2::ey(q)) * sy, qo = unsigned(q) * p32;
+            stage8(st + (kSlf + q) * NT, lfp_in + (qo + d));
+            stage8(st + (kSlg + q) * NT, lgp_in + (qo + d));
+            stage8(st + (kSlc + q) * NT, A.lcf + d);
+        }
+    } else {
+        for (int q = 0; q < Q; ++q) {
+            int qd;
+            const long long d = stream_dest(g, x, y, q, qd);
+            stage8(st + (kSlf + q) * NT, lfp_in + qd * ps + d);
+            stage8(st + (kSlg + q) * NT, lgp_in + qd * ps + d);
+            stage8(st + (kSlc + q) * NT, A.lcf + d);
+        }
     }
 }
 
@@ -239,18 +264,27 @@ __device__ __forceinline__ void prefetch_l2(const double* p) { asm volatile("pre
 // (1) node-local reverse of step k (parity par) at every interior node.  `next`: the tape
 // entry the next kernel of the sweep reads (step k - 1), whose populations are brought into
 // L2 while this step computes (null when it lies in another tape).
+//
+// Bound by latency: one thread per node is 14 warps per SM at 128 registers.  What depends on
+// the tape alone, half of the loads and the recomputed update up to its first adjoint, runs
+// before the wait for the previous kernel of the sweep.  The first kernel of a segment waits
+// first, and lets no other kernel start until then: its tape was written by kernels before it.
+// Adjoint of 200 steps of a 256x256 drop (forward and reverse): 8.43 to 8.74 ms with every load
+// after the wait and through registers, 7.83 with the tape's part before the wait, 6.95 with
+// asynchronous copies too; 64x64, 100 steps: 2.90, 2.33, 2.20.
 __global__ void __launch_bounds__(kNodeThreads, 2) adj_node_kernel(Geom g, PhysD pd, ParamChain pc, Tape in,
-                                                                   const double* c_out, AdjBufs A, int par, Tape next) {
+                                                                   const double* c_out, AdjBufs A, int par, Tape next, bool first) {
     constexpr int NT = kNodeThreads;
     extern __shared__ double stage[];  // [kStage][kNodeThreads], each thread its own column
-    chain_wait();
+    if (first) wait_for_predecessor();
+    let_successor_start();
     const int x = blockIdx.x * blockDim.x + threadIdx.x + 1, y = blockIdx.y * blockDim.y + threadIdx.y + 1;
     double pg = 0.0, psig = 0.0, pmob = 0.0;
     if (x <= g.n[0] && y <= g.n[1]) {
         const long long self = nidx(g, x, y, 0);
         const long long ps = g.ps;
         const double* st = stage + threadIdx.y * blockDim.x + threadIdx.x;
-        stage_node(g, x, y, in, c_out, A, par, stage + threadIdx.y * blockDim.x + threadIdx.x);
+        stage_tape(g, x, y, in, c_out, stage + threadIdx.y * blockDim.x + threadIdx.x);
         if (next.f) {
 #pragma unroll
             for (int q = 0; q < Q; ++q) {
@@ -258,8 +292,8 @@ __global__ void __launch_bounds__(kNodeThreads, 2) adj_node_kernel(Geom g, PhysD
                 prefetch_l2(next.g + q * ps + self);
             }
         }
-        double lc = A.lclag[self];
-        A.lclag[self] = 0.0;  // receives the ghost-layer scatter of this step (adj_c_kernel)
+        const double uprev[2] = {in.u[self], in.u[ps + self]};
+        staged();
         // stencils of c
         double lap = 0.0, dc[2] = {0.0, 0.0};
 #pragma unroll
@@ -298,7 +332,6 @@ __global__ void __launch_bounds__(kNodeThreads, 2) adj_node_kernel(Geom g, PhysD
         const double s9 = 1.0 / (tau + 0.5), kvis = -tau * pd.drho, fcap = mu - p * pd.drho3, p3 = p * (1.0 / 3.0);
         const double gfac = pd.caseType == 2 ? rho : rho - pc.rref;
         const double grav[2] = {gfac * pd.g[0], gfac * pd.g[1]};
-        const double uprev[2] = {in.u[self], in.u[ps + self]};
         Force f1, f2;
         force_fwd(uprev, Pi, p3, s9, kvis, fcap, dc, grav, f1);
         const double h = 0.5 * irho;
@@ -312,6 +345,11 @@ __global__ void __launch_bounds__(kNodeThreads, 2) adj_node_kernel(Geom g, PhysD
         const double f15 = 1.5 * irho, f15r = f15 * irho;
 
         // ---- reverse
+        wait_for_predecessor();
+        stage_adjoints(g, x, y, A, par, stage + threadIdx.y * blockDim.x + threadIdx.x);
+        double lc = A.lclag[self];
+        A.lclag[self] = 0.0;  // receives the ghost-layer scatter of this step (adj_c_kernel)
+        staged();
         double lmu = 0.0, ldcv[2] = {0.0, 0.0}, lu[2] = {A.lu[self], A.lu[ps + self]};
         double lp = 0.0, lrho = 0.0, ls9 = 0.0, lU2 = 0.0, lwc = 0.0, lamob3 = 0.0, lpref = 0.0;
         double lnrm[2] = {0.0, 0.0}, lF2[2] = {0.0, 0.0}, ldev2[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
@@ -331,7 +369,7 @@ __global__ void __launch_bounds__(kNodeThreads, 2) adj_node_kernel(Geom g, PhysD
             }
             phi *= 4.5;
             // g output
-            const double lg_q = st[(kSlg + q) * NT];
+            const double lg_q = st[(kSlg + q) * NT] + st[(kSlc + q) * NT];
             const double ga = w * (3.0 * eu + 4.5 * eu * eu - 1.5 * U2);
             const double H = c * (ga + w) + w * pref * en;
             lgp_out[q * ps + self] = lg_q * pd.one_minus_wc;
@@ -783,7 +821,7 @@ int clipb_adjoint(clipb_solver* s, const double* c0_host, int nsteps, const doub
             A.partials = partials + 3 * (size_t)nblocks * i;
             const Tape next = i > 0 ? view(tp + (size_t)(i - 1) * state) : Tape{nullptr, nullptr, nullptr, nullptr};
             CLIPB_CUDA(launch_chained(adj_node_kernel, gi, blk, kNodeSmem, s->stream, g, pd, pc, in, c_out, A,
-                                      (k0 + i) & 1, next));
+                                      (k0 + i) & 1, next, i == len - 1));
             CLIPB_CUDA(launch_chained(adj_c_kernel, gi, blk, 0, s->stream, g, A));
         }
         accumulate3<<<1, 96, 0, s->stream>>>(partials, len * nblocks, acc);

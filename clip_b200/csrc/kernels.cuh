@@ -837,9 +837,11 @@ __global__ void __launch_bounds__(256, 2) init_kernel(DevState st, int z_first) 
 // chain_wait, first in such a kernel, waits until its predecessor has completed with its
 // writes visible (griddepcontrol.wait: a hardware dependency, not a spin; after an
 // ordinary launch it returns at once).
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    let_successor_start();
+    wait_for_predecessor();
 }
 
 template <typename... P, typename... Args>

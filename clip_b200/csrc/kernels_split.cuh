@@ -8,9 +8,9 @@
 // it needs at once and the march's chain of planes is gone, for 84 bytes more per node (FP32;
 // g read a second time, c written and read).  Measured on a B200, us per step, against the
 // march at its best tile and planes per block:
-//   FP32 3D: 256x512x256 2570 / 2920, 128x256x128 341 / 428, 64x96x64 41 / 54
-//   FP64 3D: 128x256x128 1010 / 1082, 97x131x83 331 / 395, 64x96x64 97 / 137
-//   2D, FP64: 256x1024 29 / 33, 64x128 7.2 / 8.7; FP32: 201x777 11.9 / 14.2, 64x128 7.0 / 7.4
+//   FP32 3D: 256x512x256 2574 / 2921, 128x256x128 339 / 429, 64x96x64 41 / 54
+//   FP64 3D: 128x256x128 876 / 1083, 97x131x83 305 / 395, 64x96x64 93 / 137
+//   2D, FP64: 256x1024 26.5 / 33.1, 64x128 7.5 / 8.5; FP32: 201x777 10.7 / 14.1, 64x128 6.3 / 6.6
 // Cutting a 3D grid into chunks of planes, so that the second read of g comes from L2, did not
 // pay: each chunk's two launches drain the GPU (16 planes: 2.72 ms, 64: 2.66, all: 2.66).
 //
@@ -134,8 +134,6 @@ __device__ __forceinline__ void unshift(const Column<DIM, kWalls>& col, const fl
     }
 }
 
-__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // c of this step at (x, y, z), ghost coordinates included (x an interior node's: its neighbours
 // in the x ghost columns with it).

@@ -363,11 +363,12 @@ struct Launch {
 
     // Launch variant of a new solver: the two-pass step.  Measured on a B200, us per step, against
     // the best of the marching variants at its best planes or rows per block:
-    //   3D FP32: 32x48x32 13 / 19, 64x96x64 41 / 54, 97x131x83 with walls 143 / 160, 128x256x128
-    //     341 / 428, 256x512x256 2570 / 2920, 64x160x64 with inlet and outflow 117 / 217
-    //   3D FP64: 32x48x32 20 / 26, 64x96x64 92 / 137, 128x256x128 887 / 1082, 256^3 3620 / 4160
-    //   2D FP32: 64x128 6.1 / 7.4, 201x777 10.6 / 14.2, 256x1024 12.5 / 14.9, 1024x4096 158 / 171
-    //   2D FP64: 64x128 6.7 / 8.7, 201x777 19 / 27, 256x1024 28 / 33, 1024x4096 493 / 524
+    //   3D FP32: 32x48x32 12.6 / 21.7, 64x96x64 41 / 54, 97x131x83 in walls 118 / 161, 128x256x128
+    //     339 / 429, 256x512x256 2574 / 2921, 64x160x64 with inlet and outflow 129 / 215
+    //   3D FP64: 32x48x32 20 / 29, 64x96x64 93 / 137, 97x131x83 in walls 305 / 395, 128x256x128
+    //     876 / 1083, 256^3 3508 / 4173, 64x160x64 with inlet and outflow 263 / 419
+    //   2D FP32: 64x128 6.3 / 6.6, 201x777 10.7 / 14.1, 256x1024 12.5 / 14.3, 1024x4096 159 / 169
+    //   2D FP64: 64x128 7.5 / 8.5, 201x777 18.5 / 27.1, 256x1024 26.5 / 33.1, 1024x4096 455 / 552
     static constexpr int kTwoPass3 = PR::kExact ? 4 : 7, kTwoPass2 = 3;
     static int default_variant(const DevState& st) { return st.g.dim == 3 ? kTwoPass3 : kTwoPass2; }
     // whether a variant marches over `seg` planes or rows per block
