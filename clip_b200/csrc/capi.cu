@@ -473,7 +473,8 @@ static int upload_initial(clipb_solver* s, Row&& row, Uniform&& uniform_row) {
         if (jlo > jhi) return;
         for (int j = jlo; j <= jhi; ++j)  // rows inside the copied range that were not written
             if (u[j] == 2) std::fill_n(dv + s->dev_index(0, j, k), E0, rv[j]);
-        const long long a = s->dev_index(0, jlo, k), b = s->dev_index(0, jhi + 1, k);
+        // up to the next row's start, which after the last row lies beyond the array
+        const long long a = s->dev_index(0, jlo, k), b = std::min<long long>(s->dev_index(0, jhi + 1, k), g.ps);
         if (cudaMemcpyAsync(s->st.c0 + a, dv + a, (size_t)(b - a) * sizeof(double), cudaMemcpyHostToDevice, s->stream) !=
             cudaSuccess)
             copy_error.store(1);
