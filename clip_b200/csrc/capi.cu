@@ -186,7 +186,7 @@ int clipb::solver_create(const CaseConfig& cfg, int precision, clipb_solver** ou
     if ((rc = s->alloc((void**)&s->d_mon, 3 * sizeof(double)))) return rc;
     if ((rc = s->alloc((void**)&st.err, sizeof(int)))) return rc;
     // the two-pass step's work array comes last: where it does not fit, the step marches instead
-    if (s->alloc(&st.cw, (size_t)g.ps * 8)) {
+    if (s->kt.two_pass_fits(g) && s->alloc(&st.cw, (size_t)g.ps * 8)) {
         st.cw = nullptr;
         (void)cudaGetLastError();
     }

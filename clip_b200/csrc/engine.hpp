@@ -99,7 +99,8 @@ struct DevState {
     // monitor partials written by a monitored 3D step (mass and kinetic energy of each row
     // segment of 32 nodes, 2 doubles each), or null: set only for that step's launch
     double* mon_rows;
-    void* cw;            // two-pass step: c of the step (8 bytes per node); null: no memory for it
+    void* cw;            // two-pass step: c of the step (8 bytes per node); null: no memory for it,
+                         // or a grid its launches cannot cover
     double pop_scale;    // FP16: power-of-two scale of stored f
     int variant;         // launch variant of the fused step (Launch::step)
     int seg;             // planes (3D) / rows (2D) per CTA; 0 = default
@@ -129,6 +130,7 @@ struct KernelTable {
     bool (*available)(const DevState&, int variant);  // launch variant usable on this solver
     int (*default_variant)(const DevState&);
     bool (*marches)(const DevState&, int variant);  // the variant's blocks march over DevState::seg planes or rows
+    bool (*two_pass_fits)(const Geom&);             // the two-pass step's launches can cover the grid
     InitFn init;
     InitPlanesFn init_planes;  // the initial state of ghosted planes [z0, z1) only
     StepFn ghost;      // velocity-inlet ghost planes before step k (nullptr-safe: no-op without inlet)

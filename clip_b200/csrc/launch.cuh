@@ -265,7 +265,7 @@ struct Launch {
         }
     }
 
-    // The two-pass step (kernels_split.cuh).
+    // The two-pass step (kernels_split.cuh), on grids that two_pass_fits allows.
     template <int DIM, bool kOpen>
     static void go_split(const DevState& st, const StepArgs<PR>& a, cudaStream_t s) {
         if constexpr (!PR::kExact && !kOpen)
@@ -371,6 +371,16 @@ struct Launch {
     //   2D FP64: 64x128 7.5 / 8.5, 201x777 18.5 / 27.1, 256x1024 26.5 / 33.1, 1024x4096 455 / 552
     static constexpr int kTwoPass3 = PR::kExact ? 4 : 7, kTwoPass2 = 3;
     static int default_variant(const DevState& st) { return st.g.dim == 3 ? kTwoPass3 : kTwoPass2; }
+    // Whether a launch of the two-pass step can cover the grid: a launch has at most 65,535 blocks
+    // in y and in z, and its blocks hold 4 rows (3D: 8 for the phase field and FP64) of one plane.
+    // Grids beyond march with variant 0.  Launches over bands of rows would cover them too, but the
+    // band's first row as one more kernel argument cost the 128x256x128 FP16 step 4% and the
+    // 64x160x64 FP32 step with inlet and outflow 3%.
+    static bool two_pass_fits(const Geom& g) {
+        constexpr long long kMax = 65535;
+        const long long phase = g.dim == 3 ? 8 : 4, update = PR::kExact ? (g.dim == 3 ? ShapeFp64<3>::kRows : ShapeFp64<2>::kRows) : 4;
+        return g.n[1] + 2 <= kMax * phase && g.n[1] <= kMax * update && (g.dim == 2 || g.n[2] + 2 <= kMax);
+    }
     // whether a variant marches over `seg` planes or rows per block
     static bool marches(const DevState& st, int variant) { return variant != default_variant(st); }
 
@@ -451,6 +461,7 @@ struct Launch {
         t.available = &available;
         t.default_variant = &default_variant;
         t.marches = &marches;
+        t.two_pass_fits = &two_pass_fits;
         t.args_bytes = sizeof(StepArgs<PR>);
         t.make_args = &make_args;
         t.step2_batch = &step2_batch;
