@@ -722,7 +722,12 @@ int clipb_autotune(clipb_solver* s, int trial_steps, int* best_variant, int* bes
         for (size_t i = 0; i < cands.size(); ++i) {
             const size_t c = pass == 0 ? i : cands.size() - 1 - i;
             if ((rc = clipb_set_launch(s, cands[c].first, cands[c].second))) return rc;
-            if ((rc = clipb_solve(s, 1))) return rc;  // warm-up
+            // warm-up; a shape with more blocks in y than a launch holds is not a candidate
+            CLIPB_CUDA(s->kt.ghost(s->st, s->steps, s->stream));
+            const cudaError_t e = s->kt.step(s->st, s->steps, s->stream);
+            if (e == cudaErrorInvalidConfiguration) continue;
+            CLIPB_CUDA(e);
+            ++s->steps;
             float ms = 0.f;
             if ((rc = clipb_time_steps(s, trial_steps, &ms))) return rc;
             ms_best[c] = std::min(ms_best[c], ms);

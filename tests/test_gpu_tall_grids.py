@@ -62,3 +62,16 @@ def test_planes(tmp_path, prec, nz):
     # fields of more than 65,535 planes cannot be read back: their sums are compared
     path = _tall(tmp_path / "config.txt", (2, 2, nz), "ppw", 2, min(nz - 2, 65536))
     _same(path, prec, 2 if prec == "fp64" else 8, 4 if prec == "fp64" else 7, ("c", "vel", "g") if nz <= 65533 else (), True)
+
+
+@pytest.mark.parametrize("ny", [70000, 262200])
+def test_autotune_skips_shapes_that_a_launch_cannot_cover(tmp_path, ny):
+    """One row per block is such a shape on both grids."""
+    with cb.Solver(_tall(tmp_path / "config.txt", (2, ny), "pw", 1, ny // 2), "fp32") as s:
+        s.init()
+        want = s.interior_field("c")
+        variant, seg, ms = s.autotune(2)
+        assert ms < 1e6 and (variant == 3 or seg > 1)
+        assert s.steps == 0 and np.array_equal(s.interior_field("c"), want)
+        s.solve(3)
+        assert np.isfinite(s.interior_field("c")).all()
