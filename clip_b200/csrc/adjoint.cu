@@ -251,9 +251,9 @@ int clipb_tangent(clipb_solver* s, const double* c0_host, int nsteps, const doub
     const size_t ps = (size_t)g.ps;
     DevVec mem, c0v, c0d;
     const size_t nd = 4 * Q * ps + 2 * ps + 2 * ps;
-    cudaError_t e = mem.alloc(nd * sizeof(Dual));
-    if (e == cudaSuccess) e = c0v.alloc(ps * sizeof(double));
-    if (e == cudaSuccess) e = c0d.alloc(ps * sizeof(double));
+    cudaError_t e = mem.alloc(s, nd * sizeof(Dual));
+    if (e == cudaSuccess) e = c0v.alloc(s, ps * sizeof(double));
+    if (e == cudaSuccess) e = c0d.alloc(s, ps * sizeof(double));
     if (e != cudaSuccess) return fail(CLIPB_E_NOMEM, std::string("tangent-linear buffers: ") + cudaGetErrorString(e));
     CLIPB_CUDA(cudaMemcpy(c0v.p, cv.data(), ps * sizeof(double), cudaMemcpyHostToDevice));
     CLIPB_CUDA(cudaMemcpy(c0d.p, cd.data(), ps * sizeof(double), cudaMemcpyHostToDevice));

@@ -59,8 +59,8 @@ inline ParamChain chain(const PhysD& d) {
 struct DevVec {  // owned device allocation
     void* p = nullptr;
     ~DevVec() { cudaFree(p); }
-    cudaError_t alloc(size_t bytes) {
-        cudaError_t e = cudaMalloc(&p, bytes);
+    cudaError_t alloc(clipb_solver* s, size_t bytes) {
+        cudaError_t e = s->device_malloc(&p, bytes);
         if (e == cudaSuccess) e = cudaMemset(p, 0, bytes);
         return e;
     }

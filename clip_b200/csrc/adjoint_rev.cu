@@ -668,7 +668,7 @@ int ensure_work(clipb_solver* s, size_t bytes) {
     if (w->mem) cudaFree(w->mem);
     w->mem = nullptr;
     w->bytes = 0;
-    const cudaError_t e = cudaMalloc(&w->mem, bytes);
+    const cudaError_t e = s->device_malloc(&w->mem, bytes);
     if (e != cudaSuccess)
         return fail(CLIPB_E_NOMEM, "adjoint workspace of " + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e) +
                                        " (a smaller checkpoint interval needs less)");
@@ -694,10 +694,10 @@ int clipb_adjoint(clipb_solver* s, const double* c0_host, int nsteps, const doub
     int K = checkpoint_every;
     if (K <= 0) {
         // every state of the run in one tape (no recomputation) when the tape takes at most
-        // half of the device memory that is free, counting the workspace this solver holds
+        // half of the device memory that is free, counting the workspaces this solver holds
         size_t free_b = 0, total_b = 0;
         CLIPB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        const size_t held = s->adjw ? s->adjw->bytes : 0;
+        const size_t held = (s->adjw ? s->adjw->bytes : 0) + (s->st.cw ? s->work_bytes() : 0);
         K = ((size_t)nsteps + 1) * state * sizeof(double) <= (free_b + held) / 2 ? nsteps : 100;
     }
     const int nck = (nsteps + K - 1) / K, last = nck - 1, len_last = nsteps - last * K;

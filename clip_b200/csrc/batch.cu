@@ -60,40 +60,77 @@ struct clipb_batch {
 
 namespace {
 
-// Whether every case can run the variant (the FP32/FP16 two-pass step needs its work arrays).
+// Whether every case can run the variant.
 bool launchable(const clipb_batch* b, int variant) {
-    for (const auto* c : b->cases) {
+    for (const auto* c : b->cases)
         if (!b->kt.available(c->st, variant)) return false;
-        if (b->precision != CLIPB_FP64 && variant == b->kt.default_variant(c->st) && !c->st.cw) return false;
-    }
     return true;
 }
+// The launch variant that runs when `variant` is asked for: without the work arrays of all cases
+// variant 0 marches in the two-pass step's place.
+int launch_variant(const clipb_batch* b, int variant) {
+    if (!b->kt.two_pass_batch(variant)) return variant;
+    for (const auto* c : b->cases)
+        if (!c->st.cw) return 0;
+    return variant;
+}
 
-// Work items (case, tile bx, row segment by) for a tile width and segment length, case by
-// case so that CTAs running at the same time work on neighbouring tiles of one case.
-int build_items(clipb_batch* b) {
-    const int TX = b->kt.tile2(b->variant);
-    std::vector<int> items;
-    for (size_t c = 0; c < b->cases.size(); ++c) {
-        const Geom& g = b->cases[c]->st.g;
-        const int nbx = (g.n[0] + TX - 1) / TX, nby = (g.n[1] + b->seg - 1) / b->seg;
-        for (int by = 0; by < nby; ++by)
-            for (int bx = 0; bx < nbx; ++bx) {
-                items.push_back((int)c);
-                items.push_back(bx);
-                items.push_back(by);
-            }
+// cudaMalloc of the batch's own buffers, the cases' work arrays given back where memory is short.
+cudaError_t batch_malloc(clipb_batch* b, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        for (auto* c : b->cases) c->drop_work();
+        e = cudaMalloc(p, bytes);
     }
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+}
+
+// Sets the launch shape and its work items (case, tile bx, row segment by), case by case so that
+// CTAs running at the same time work on neighbouring tiles of one case.
+int build_items(clipb_batch* b, int variant, int seg) {
     CLIPB_CUDA(cudaStreamSynchronize(b->stream));
+    b->drop_graph();
     cudaFree(b->d_items);
     b->d_items = nullptr;
-    CLIPB_CUDA(cudaMalloc((void**)&b->d_items, items.size() * sizeof(int)));
+    b->nitems = 0;
+    std::vector<int> items;
+    for (bool again = true; again;) {
+        again = false;
+        b->variant = launch_variant(b, variant);
+        b->seg = seg;
+        const int TX = b->kt.tile2(b->variant);
+        items.clear();
+        for (size_t c = 0; c < b->cases.size(); ++c) {
+            const Geom& g = b->cases[c]->st.g;
+            const int nbx = (g.n[0] + TX - 1) / TX, nby = (g.n[1] + seg - 1) / seg;
+            for (int by = 0; by < nby; ++by)
+                for (int bx = 0; bx < nbx; ++bx) {
+                    items.push_back((int)c);
+                    items.push_back(bx);
+                    items.push_back(by);
+                }
+        }
+        CLIPB_CUDA(batch_malloc(b, (void**)&b->d_items, items.size() * sizeof(int)));
+        if (launch_variant(b, b->variant) != b->variant) {  // the work arrays made room for the items
+            cudaFree(b->d_items);
+            b->d_items = nullptr;
+            again = true;
+        }
+    }
     CLIPB_CUDA(cudaMemcpy(b->d_items, items.data(), items.size() * sizeof(int), cudaMemcpyHostToDevice));
     b->nitems = (int)(items.size() / 3);
     return CLIPB_OK;
 }
 
+// Whether the launch shape is set: not after an allocation of its items failed.
+int check_items(const clipb_batch* b) {
+    return b->nitems ? CLIPB_OK : fail(CLIPB_E_NOMEM, "the batch has no work items: set its launch shape again");
+}
+
 int launch_batched(clipb_batch* b) {
+    if (const int rc = check_items(b)) return rc;
     CLIPB_CUDA(b->kt.step2_batch(b->d_args[b->steps & 1], b->d_items, b->nitems, b->variant, b->seg,
                                  b->blocks_per_sm, b->stream));
     ++b->steps;
@@ -102,6 +139,7 @@ int launch_batched(clipb_batch* b) {
 }
 
 int build_graph(clipb_batch* b) {
+    if (const int rc = check_items(b)) return rc;
     cudaGraph_t g = nullptr;
     CLIPB_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     for (int i = 0; i < clipb_batch::kGraphSteps; ++i) {
@@ -151,6 +189,11 @@ std::string seeded_config(uint64_t seed, int index) {
 
 }  // namespace
 
+void clipb::batch_drop_work(clipb_batch* b) {
+    for (auto* c : b->cases) c->drop_work();
+    if (b->nitems && launch_variant(b, b->variant) != b->variant) (void)build_items(b, b->variant, b->seg);
+}
+
 extern "C" {
 
 int clipb_seeded_case_config(unsigned long long seed, int index, char* buf, size_t len) {
@@ -186,31 +229,34 @@ int clipb_batch_create(const char* const* configs, int ncases, int kind, int pre
                 return fail(CLIPB_E_CONFIG, "case " + std::to_string(i) +
                                                 ": batched cases take wall, slip-wall and periodic sides");
         clipb_solver* s = nullptr;
-        const int rc = solver_create(cfg, precision, &s);
+        int rc = solver_create(cfg, precision, &s);
+        if (rc == CLIPB_E_NOMEM) {  // the work arrays of the cases before make room
+            for (auto* c : b->cases) c->drop_work();
+            rc = solver_create(cfg, precision, &s);
+        }
         if (rc) return fail(rc, "case " + std::to_string(i) + ": " + clipb_last_error());
         b->cases.push_back(s);
+        s->batch = b.get();
         CLIPB_CUDA(cudaStreamSynchronize(s->stream));
         s->stream = b->stream;  // every case runs on the batch's stream
     }
     b->kt = b->cases[0]->kt;
-    if (precision != CLIPB_FP64 && launchable(b.get(), b->kt.default_variant(b->cases[0]->st))) {
-        // the two-pass step (its rates: update_batch_kernel)
-        b->variant = b->kt.default_variant(b->cases[0]->st);
-        b->seg = 16;
-    }
     // step arguments of every case for both buffer parities
     const size_t ab = b->kt.args_bytes;
     std::vector<unsigned char> host(ab * ncases);
     for (int p = 0; p < 2; ++p) {
         for (int i = 0; i < ncases; ++i) b->kt.make_args(b->cases[i]->st, p, host.data() + ab * i);
-        CLIPB_CUDA(cudaMalloc(&b->d_args[p], host.size()));
+        CLIPB_CUDA(batch_malloc(b.get(), &b->d_args[p], host.size()));
         CLIPB_CUDA(cudaMemcpy(b->d_args[p], host.data(), host.size(), cudaMemcpyHostToDevice));
     }
-    CLIPB_CUDA(cudaMalloc((void**)&b->d_mon, 3 * sizeof(double) * ncases));
+    CLIPB_CUDA(batch_malloc(b.get(), (void**)&b->d_mon, 3 * sizeof(double) * ncases));
     b->h_mon.resize(3 * (size_t)ncases);
     CLIPB_CUDA(cudaEventCreate(&b->ev0));
     CLIPB_CUDA(cudaEventCreate(&b->ev1));
-    int rc = build_items(b.get());
+    // the two-pass step where it is one (its rates: update_batch_kernel)
+    const int two_pass = b->kt.two_pass_variant(b->cases[0]->st);
+    const bool runs = b->kt.two_pass_batch(two_pass) && launch_variant(b.get(), two_pass) == two_pass;
+    const int rc = runs ? build_items(b.get(), two_pass, 16) : build_items(b.get(), 0, 8);
     if (rc) return rc;
     *out = b.release();
     return CLIPB_OK;
@@ -283,12 +329,8 @@ int clipb_batch_set_launch(clipb_batch* b, int variant, int seg, int blocks_per_
         return fail(CLIPB_E_ARG, "variant must be in [0, " + std::to_string(b->kt.variants2) + ")");
     if (seg < 1) return fail(CLIPB_E_ARG, "rows per work item must be positive");
     if (blocks_per_sm < 0) return fail(CLIPB_E_ARG, "negative blocks per SM");
-    CLIPB_CUDA(cudaStreamSynchronize(b->stream));
-    b->drop_graph();
-    b->variant = variant;
-    b->seg = seg;
     b->blocks_per_sm = blocks_per_sm;
-    return build_items(b);
+    return build_items(b, variant, seg);
 }
 
 int clipb_batch_get_launch(const clipb_batch* b, int* variant, int* seg, int* blocks_per_sm, int* nitems) {
@@ -335,10 +377,10 @@ int clipb_batch_autotune(clipb_batch* b, int trial_steps, int* best_variant, int
     float best = 1e30f;
     int bv = b->variant, bs = b->seg, bb = b->blocks_per_sm, rc;
     for (int v = 0; v < b->kt.variants2; ++v) {
-        if (!launchable(b, v)) continue;
+        if (!launchable(b, v) || launch_variant(b, v) != v) continue;
         for (int seg : {4, 8, 16, 32, 64})
             for (int bps : {1, 2, 0}) {
-                if (bps && b->precision != CLIPB_FP64 && !b->kt.marches(b->cases[0]->st, v)) continue;  // not persistent
+                if (bps && b->kt.two_pass_batch(v)) continue;  // not persistent
                 if ((rc = clipb_batch_set_launch(b, v, seg, bps))) return rc;
                 if ((rc = clipb_batch_solve(b, 1))) return rc;  // warm-up
                 float ms = 0.f;

@@ -148,7 +148,6 @@ int clipb::solver_create(const CaseConfig& cfg, int precision, clipb_solver** ou
     }
     s->kt = precision == CLIPB_FP64 ? kernels_fp64() : (precision == CLIPB_FP32 ? kernels_fp32() : kernels_fp16());
     st.seg = 0;
-    st.variant = s->kt.default_variant(st);  // clipb_autotune can pick another one
 
     const int Q = c.dim == 3 ? 19 : 9;
     // the step kernels index every buffer with 32-bit element offsets
@@ -186,10 +185,8 @@ int clipb::solver_create(const CaseConfig& cfg, int precision, clipb_solver** ou
     if ((rc = s->alloc((void**)&s->d_mon, 3 * sizeof(double)))) return rc;
     if ((rc = s->alloc((void**)&st.err, sizeof(int)))) return rc;
     // the two-pass step's work array comes last: where it does not fit, the step marches instead
-    if (s->kt.two_pass_fits(g) && s->alloc(&st.cw, (size_t)g.ps * 8)) {
-        st.cw = nullptr;
-        (void)cudaGetLastError();
-    }
+    if (s->kt.two_pass_fits(g) && s->alloc(&st.cw, s->work_bytes())) st.cw = nullptr;
+    st.variant = s->launch_variant(s->kt.two_pass_variant(st));  // clipb_autotune can pick another one
     CLIPB_CUDA(cudaMallocHost((void**)&s->h_mon, 4 * sizeof(double)));  // the last one: the wait flag
     // staged variants need tensor maps of the buffers; without them they are unavailable
     if (s->kt.prepare(st) != cudaSuccess) {
@@ -659,7 +656,7 @@ int clipb_set_launch(clipb_solver* s, int variant, int seg) {
         return fail(CLIPB_E_ARG, "variant " + std::to_string(variant) + " is unavailable on this solver");
     if (seg < 0) return fail(CLIPB_E_ARG, "negative segment length");
     CLIPB_CUDA(cudaStreamSynchronize(s->stream));
-    s->st.variant = variant;
+    s->st.variant = s->launch_variant(variant);
     s->st.seg = seg;
     s->drop_graph();
     return CLIPB_OK;
@@ -713,9 +710,9 @@ int clipb_autotune(clipb_solver* s, int trial_steps, int* best_variant, int* bes
     // so that a drift favours none of them.
     std::vector<std::pair<int, int>> cands;
     for (int v = 0; v < nv; ++v) {
-        if (!s->kt.available(s->st, v)) continue;
+        if (!s->kt.available(s->st, v) || s->launch_variant(v) != v) continue;
         for (int seg : segs)
-            if (seg == segs.front() || (seg <= n_march && s->kt.marches(s->st, v))) cands.emplace_back(v, seg);
+            if (seg == segs.front() || (seg <= n_march && !s->kt.two_pass(s->st, v))) cands.emplace_back(v, seg);
     }
     std::vector<float> ms_best(cands.size(), 1e30f);
     for (int pass = 0; pass < 2; ++pass) {

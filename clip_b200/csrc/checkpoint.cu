@@ -219,7 +219,7 @@ int clipb_load(clipb_solver* s, const char* dir) {
     }
     double* d = nullptr;
     const size_t pq = nodes * Q;
-    CLIPB_CUDA(cudaMalloc((void**)&d, (2 * pq + nodes + nodes * dim) * sizeof(double)));
+    CLIPB_CUDA(s->device_malloc((void**)&d, (2 * pq + nodes + nodes * dim) * sizeof(double)));
     auto upload = [&](size_t off, const std::vector<double>& v) {
         return cudaMemcpyAsync(d + off, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, s->stream);
     };

@@ -100,7 +100,7 @@ struct DevState {
     // segment of 32 nodes, 2 doubles each), or null: set only for that step's launch
     double* mon_rows;
     void* cw;            // two-pass step: c of the step (8 bytes per node); null: no memory for it,
-                         // or a grid its launches cannot cover
+                         // or a grid its launches cannot cover.  `variant` is then not the two-pass one
     double pop_scale;    // FP16: power-of-two scale of stored f
     int variant;         // launch variant of the fused step (Launch::step)
     int seg;             // planes (3D) / rows (2D) per CTA; 0 = default
@@ -128,9 +128,10 @@ struct KernelTable {
     cudaError_t (*prepare)(DevState&);
     void (*release)(DevState&);
     bool (*available)(const DevState&, int variant);  // launch variant usable on this solver
-    int (*default_variant)(const DevState&);
-    bool (*marches)(const DevState&, int variant);  // the variant's blocks march over DevState::seg planes or rows
-    bool (*two_pass_fits)(const Geom&);             // the two-pass step's launches can cover the grid
+    int (*two_pass_variant)(const DevState&);
+    bool (*two_pass)(const DevState&, int variant);  // else the variant's blocks march over DevState::seg planes or rows
+    bool (*two_pass_batch)(int variant);             // the same of a batch's step
+    bool (*two_pass_fits)(const Geom&);              // the two-pass step's launches can cover the grid
     InitFn init;
     InitPlanesFn init_planes;  // the initial state of ghosted planes [z0, z1) only
     StepFn ghost;      // velocity-inlet ghost planes before step k (nullptr-safe: no-op without inlet)

@@ -235,7 +235,7 @@ struct Launch {
             default: return go2_batch<64, kKeepG2>(args, items, nitems, seg, blocks_per_sm, s);
         }
     }
-    static int tile2(int variant) { return variant == 1 || (!PR::kExact && variant == 3) ? 32 : (variant == 2 ? 128 : 64); }
+    static int tile2(int variant) { return variant == 1 || two_pass_batch(variant) ? 32 : (variant == 2 ? 128 : 64); }
     static void make_args(const DevState& st, long long k, void* out) {
         const StepArgs<PR> a = args(st, k);
         std::memcpy(out, &a, sizeof(a));
@@ -325,10 +325,8 @@ struct Launch {
     // kOpen: the kernel instances for cases with free-convect or Neumann sides.
     template <bool kOpen>
     static void step_shape(const DevState& st, const StepArgs<PR>& a, long long k, cudaStream_t s) {
-        // without its work array the two-pass step's variant is the march of variant 0
-        const int variant = !st.cw && st.variant == default_variant(st) ? 0 : st.variant;
         if (st.g.dim == 3) {
-            switch (variant) {
+            switch (st.variant) {
                 case 1: go3<32, 8, kKeepG3, kOpen>(st, a, s); break;
                 case 2: go3<32, 16, false, kOpen>(st, a, s); break;
                 case 3: go3<64, 8, false, kOpen>(st, a, s); break;
@@ -352,7 +350,7 @@ struct Launch {
                 default: go3<32, 8, false, kOpen>(st, a, s); break;
             }
         } else {
-            switch (variant) {
+            switch (st.variant) {
                 case 1: go2<32, kKeepG2, kOpen>(st, a, s); break;
                 case 2: go2<128, kKeepG2, kOpen>(st, a, s); break;
                 case 3: go_split<2, kOpen>(st, a, s); break;
@@ -370,7 +368,9 @@ struct Launch {
     //   2D FP32: 64x128 6.3 / 6.6, 201x777 10.7 / 14.1, 256x1024 12.5 / 14.3, 1024x4096 159 / 169
     //   2D FP64: 64x128 7.5 / 8.5, 201x777 18.5 / 27.1, 256x1024 26.5 / 33.1, 1024x4096 455 / 552
     static constexpr int kTwoPass3 = PR::kExact ? 4 : 7, kTwoPass2 = 3;
-    static int default_variant(const DevState& st) { return st.g.dim == 3 ? kTwoPass3 : kTwoPass2; }
+    static int two_pass_variant(const DevState& st) { return st.g.dim == 3 ? kTwoPass3 : kTwoPass2; }
+    static bool two_pass(const DevState& st, int variant) { return variant == two_pass_variant(st); }
+    static bool two_pass_batch(int variant) { return !PR::kExact && variant == kTwoPass2; }
     // Whether a launch of the two-pass step can cover the grid: a launch has at most 65,535 blocks
     // in y and in z, and its blocks hold 4 rows (3D: 8 for the phase field and FP64) of one plane.
     // Grids beyond march with variant 0.  Launches over bands of rows would cover them too, but the
@@ -381,8 +381,6 @@ struct Launch {
         const long long phase = g.dim == 3 ? 8 : 4, update = PR::kExact ? (g.dim == 3 ? ShapeFp64<3>::kRows : ShapeFp64<2>::kRows) : 4;
         return g.n[1] + 2 <= kMax * phase && g.n[1] <= kMax * update && (g.dim == 2 || g.n[2] + 2 <= kMax);
     }
-    // whether a variant marches over `seg` planes or rows per block
-    static bool marches(const DevState& st, int variant) { return variant != default_variant(st); }
 
     static cudaError_t step(const DevState& st, long long k, cudaStream_t s) {
         const StepArgs<PR> a = args(st, k);
@@ -459,8 +457,9 @@ struct Launch {
         t.prepare = &prepare;
         t.release = &release;
         t.available = &available;
-        t.default_variant = &default_variant;
-        t.marches = &marches;
+        t.two_pass_variant = &two_pass_variant;
+        t.two_pass = &two_pass;
+        t.two_pass_batch = &two_pass_batch;
         t.two_pass_fits = &two_pass_fits;
         t.args_bytes = sizeof(StepArgs<PR>);
         t.make_args = &make_args;

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <memory>
 #include <string>
 #include <vector>
@@ -21,6 +22,8 @@ void vts_release(VtsQueue* q);
 // Device workspace of clipb_adjoint (adjoint_rev.cu), kept for later calls.
 struct AdjWork;
 void adj_release(AdjWork* w);
+// drop_work of every case of a batch, which marches from then on (batch.cu).
+void batch_drop_work(clipb_batch* b);
 }  // namespace clipb
 
 #define CLIPB_CUDA(call)                                                                                      \
@@ -75,6 +78,7 @@ struct clipb_solver {
     bool use_graphs = true;
     clipb::VtsQueue* vts = nullptr;  // created by the first VTS write
     clipb::AdjWork* adjw = nullptr;  // created by the first clipb_adjoint
+    clipb_batch* batch = nullptr;    // the batch whose case this is
     bool slab_half = false;          // a slab step's first part ran (clipb_slab_step_part)
     size_t fc_bytes = 0;             // bytes of each parity's free-convect state (st.g.fc)
 
@@ -96,8 +100,36 @@ struct clipb_solver {
     // element index of reference node (i, j, k) in the device layout
     long long dev_index(int i, int j, int k) const { return st.g.base + i + (long long)j * st.g.sy + (long long)k * st.g.sz; }
 
+    // cudaMalloc.  Where memory is short, the two-pass step's work array, which no call depends on,
+    // is given back first (a batch's case: those of all its cases).
+    cudaError_t device_malloc(void** p, size_t bytes) {
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation && (st.cw || batch)) {
+            (void)cudaGetLastError();
+            if (batch) clipb::batch_drop_work(batch);
+            else drop_work();
+            e = cudaMalloc(p, bytes);
+        }
+        if (e != cudaSuccess) (void)cudaGetLastError();
+        return e;
+    }
+    // Frees the work array: from now on the solver marches with variant 0 in the two-pass step's place.
+    void drop_work() {
+        if (!st.cw) return;
+        cudaStreamSynchronize(stream);
+        drop_graph();  // its launches hold the array
+        cudaFree(st.cw);
+        allocations.erase(std::remove(allocations.begin(), allocations.end(), st.cw), allocations.end());
+        device_bytes -= work_bytes();
+        st.cw = nullptr;
+        st.variant = launch_variant(st.variant);
+    }
+    size_t work_bytes() const { return (size_t)st.g.ps * 8; }
+    // the launch variant that runs when `variant` is asked for
+    int launch_variant(int variant) const { return !st.cw && kt.two_pass(st, variant) ? 0 : variant; }
+
     int alloc(void** p, size_t bytes) {
-        const cudaError_t e = cudaMalloc(p, bytes);
+        const cudaError_t e = device_malloc(p, bytes);
         if (e != cudaSuccess) return clipb::fail(CLIPB_E_NOMEM, "cudaMalloc of " + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e));
         allocations.push_back(*p);
         device_bytes += bytes;

@@ -384,7 +384,7 @@ int clipb_write_vts_async(clipb_solver* s, const char* folder, const char* base_
         if (sl.host) cudaFreeHost(sl.host);
         sl.dev = sl.host = nullptr;
         sl.bytes = 0;
-        if (cudaMalloc(&sl.dev, bytes) != cudaSuccess || cudaMallocHost(&sl.host, bytes) != cudaSuccess) {
+        if (s->device_malloc(&sl.dev, bytes) != cudaSuccess || cudaMallocHost(&sl.host, bytes) != cudaSuccess) {
             cudaGetLastError();
             return release(fail(CLIPB_E_NOMEM, "VTS buffers of " + std::to_string(bytes) + " bytes"));
         }

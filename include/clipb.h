@@ -186,9 +186,11 @@ int clipb_time_steps(clipb_solver* s, int nsteps, float* ms);
  * policy of the marching one (0 .. nvariants-1), `seg` the planes (3D) or rows (2D) each
  * thread block marches over (0 = default: 2D takes the longest of 16, 8, 4, 2 rows that
  * leaves eight blocks per SM).  The two-pass step (variant 7 in 3D FP32/FP16, 4 in 3D FP64,
- * 3 in 2D; a new solver's default) ignores seg; it keeps c of the step in 8 more bytes per
- * node, and a solver created without room for them marches with variant 0 instead.  Results
- * do not depend on the launch shape.  No reference counterpart
+ * 3 in 2D; a new solver's default) ignores seg; it keeps c of the step in a work array of 8
+ * more bytes per node.  Where variant 0 marches in its place, get_launch says so: on a solver
+ * created without room for that array, on one that gave it back to a later allocation of its
+ * own, and on grids taller than its launches (more than 262,138 rows; 65,533 planes).
+ * Results do not depend on the launch shape.  No reference counterpart
  * (the reference launches fixed 8x8(x4) blocks, DataArray.cu:27-44). */
 int clipb_set_launch(clipb_solver* s, int variant, int seg);
 int clipb_get_launch(const clipb_solver* s, int* variant, int* seg, int* nvariants);
@@ -391,7 +393,8 @@ int clipb_batch_solve_sequential(clipb_batch* b, int nsteps);
 
 /* Launch shape of the batched step: 2D tile variant (as clipb_set_launch), rows per work
  * item, persistent thread blocks per SM (0: as many as fit).  FP32/FP16 variant 3, the
- * default there, is the two-pass step: one block per work item, blocks_per_sm unused.
+ * default there, is the two-pass step: one block per work item, blocks_per_sm unused; variant 0
+ * marches in its place where a case has no work array (see clipb_set_launch).
  * Results do not depend on it. */
 int clipb_batch_set_launch(clipb_batch* b, int variant, int rows_per_item, int blocks_per_sm);
 int clipb_batch_get_launch(const clipb_batch* b, int* variant, int* rows_per_item, int* blocks_per_sm, int* nitems);
