@@ -756,6 +756,7 @@ static int ensure_stage(clipb_solver* s, size_t elems) {
         cudaFree(s->d_stage);
         s->allocations.erase(std::remove(s->allocations.begin(), s->allocations.end(), (void*)s->d_stage), s->allocations.end());
         s->d_stage = nullptr;
+        s->stage_elems = 0;
     }
     const int rc = s->alloc((void**)&s->d_stage, elems * sizeof(double));
     if (rc) return rc;

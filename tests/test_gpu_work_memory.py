@@ -78,6 +78,18 @@ def test_a_solvers_later_allocations_fit(tmp_path, call):
         assert s.get_launch()[:2] == (0, 4)
 
 
+def test_a_read_after_a_read_that_did_not_fit(tmp_path):
+    """The larger read frees the stage before it asks for its own; the next one needs a stage too."""
+    with cb.Solver(_config(tmp_path / "config.txt", (2048, 2048), "pw"), "fp32") as s:
+        s.init()
+        s.solve(2)
+        want = s.field("c")
+        with _full_but(4 * MB):
+            with pytest.raises(cb.ClipError, match="out of memory"):
+                s.field("g_post")
+            assert np.array_equal(s.field("c"), want)
+
+
 def _batch(tmp_path, prec):
     paths = [_config(tmp_path / f"config{i}.txt", (1024, 1024 + 32 * i), "pw") for i in range(4)]
     return cb.Batch([open(p).read() for p in paths], prec, texts=True)
