@@ -162,8 +162,9 @@ __device__ __forceinline__ void equilibria(T ux, T uy, T uz, T U2, T* eq) {
 // by rho); as general divisions they and their range checks were over half of its 8,800
 // instructions.  With these forms and the pairs' shared terms the 128x256x128 step went from
 // 1390 to 1082 us (32 x 16 tile), the 256x1024 2D step from 53 to 33 us.  Both forms below
-// return the correctly rounded quotient, the bits of a / b, for operands whose products stay
-// clear of underflow and overflow; callers check that with in_range and divide otherwise.
+// return the correctly rounded quotient, the bits of a / b but for the sign of a zero (that of
+// -0 / b may be +0), for operands whose products stay clear of underflow and overflow and a b
+// other than zero; callers check that with in_range and divide otherwise.
 //
 // By a constant D = 2^k 3^m, m <= 2: with hi + lo = 1/D to twice the precision, x hi + x lo is
 // off the quotient by less than 2^-50 of a unit in the last place before its one rounding, while
@@ -191,11 +192,16 @@ __device__ __forceinline__ double quotient(double a, double b, double y) {
     q = __fma_rn(__fma_rn(-b, q, a), y, q);
     return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
-// x is zero or has 2^-E <= |x| < 2^E.
+// 2^-E <= |x| < 2^E
+template <int E>
+__device__ __forceinline__ bool nonzero_in_range(double x) {
+    const unsigned t = unsigned(__double2hiint(x)) & 0x7fffffffu;
+    return t - (unsigned(1023 - E) << 20) < (unsigned(2 * E) << 20);
+}
+// The same, or zero.
 template <int E>
 __device__ __forceinline__ bool in_range(double x) {
-    const unsigned t = unsigned(__double2hiint(x)) & 0x7fffffffu;
-    return t - (unsigned(1023 - E) << 20) < (unsigned(2 * E) << 20) || x == 0.0;
+    return nonzero_in_range<E>(x) || x == 0.0;
 }
 // The update's quotients may take these forms when every f is zero or within 2^+-500, every
 // velocity component zero or within 2^+-200, and (for the collision, and for the quotients of
@@ -218,7 +224,7 @@ __device__ __forceinline__ bool all_in_range(const T* v) {
 template <int N, typename T>
 __device__ __forceinline__ void divide_all(T* a, T b, bool in) {
     if constexpr (std::is_same<T, double>::value) {
-        if (in && in_range<100>(b)) {
+        if (in && nonzero_in_range<100>(b)) {
             const double y = 1.0 / b;
 #pragma unroll
             for (int i = 0; i < N; ++i) a[i] = quotient(a[i], b, y);
