@@ -287,8 +287,10 @@ struct Launch {
         constexpr int TY = PR::kExact ? ShapeFp64<DIM>::kRows : 4;
         const int nx = (g.n[0] + 31) / 32, nz = DIM == 3 ? g.zhi - g.zlo + 1 : 1;
         const int py = DIM == 3 ? 8 : 4;  // rows per block of the phase field
-        (void)launch_chained(phase_kernel<DIM, PR, kOpen, kWalls>, dim3(nx, (g.n[1] + 2 + py - 1) / py, DIM == 3 ? nz + 2 : 1), dim3(32, py),
-                             0, s, a, ptr, g.zlo - 1);
+        // no update from a stale work array; step() reads the error
+        if (launch_chained(phase_kernel<DIM, PR, kOpen, kWalls>, dim3(nx, (g.n[1] + 2 + py - 1) / py, DIM == 3 ? nz + 2 : 1), dim3(32, py),
+                           0, s, a, ptr, g.zlo - 1) != cudaSuccess)
+            return;
         const dim3 gu(nx, (g.n[1] + TY - 1) / TY, nz), bu(32, TY);
         auto update = [&](auto mon) {
             constexpr bool kMon = decltype(mon)::value;
