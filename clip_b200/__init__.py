@@ -391,7 +391,7 @@ def seeded_case_config(seed, index):
 
 
 class Batch:
-    """Many independent 2D cases advanced together by one persistent launch per step."""
+    """Many independent 2D cases advanced together, by two launches per step (marching variants: one)."""
 
     def __init__(self, configs, precision="fp32", texts=False):
         L = load_library()

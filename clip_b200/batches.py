@@ -1,7 +1,7 @@
 """Batches of independent 2D cases over several GPUs, one process per GPU.
 
 The cases share nothing, so the case table is partitioned.  Each rank advances its own
-cases in one libclipb batch (clipb_batch_*: one persistent launch per step), and the only
+cases in one libclipb batch (clipb_batch_*: one or two launches per step), and the only
 collective is the gather of the per-case monitors at the end.  The partition balances the
 interior nodes per rank: the largest case goes first onto the least loaded rank, so the
 ranks finish a step at about the same time.  No counterpart in the reference, which runs

@@ -140,10 +140,10 @@ struct KernelTable {
     InteriorFn interior;
     MonitorFn monitors;
     MonitorRowsFn monitor_rows;
-    // launch variant whose step can write monitor partials (the 3D direct-load kernels)
+    // launch variant whose step can write monitor partials (3D, all but the staged ones)
     bool (*fused_monitors)(const DevState&);
     VtsPackFn vts_pack;
-    // batched 2D step (many cases, one persistent launch; see step2d_batch_kernel)
+    // batched 2D step of many cases (update_batch_kernel; marching variants: step2d_batch_kernel)
     size_t args_bytes;                                          // bytes of one case's step arguments
     void (*make_args)(const DevState&, long long step, void* out);  // host: arguments of step `step`
     cudaError_t (*step2_batch)(const void* args, const int* items, int nitems, int variant, int seg,

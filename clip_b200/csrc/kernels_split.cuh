@@ -5,12 +5,13 @@
 // The one-pass kernels (step2d_body, step3d_body) compute c on a tile and its halo while they
 // march, so a node's g is pulled up to 1.7 times and each plane waits for memory twice and for
 // a barrier, one plane after the other.  Here every node is independent: a block asks for all
-// it needs at once and the march's chain of planes is gone, for 84 bytes more per node (FP32;
-// g read a second time, c written and read).  Measured on a B200, us per step, against the
-// march at its best tile and planes per block:
-//   FP32 3D: 256x512x256 2574 / 2921, 128x256x128 339 / 429, 64x96x64 41 / 54
-//   FP64 3D: 128x256x128 876 / 1083, 97x131x83 305 / 395, 64x96x64 93 / 137
-//   2D, FP64: 256x1024 26.5 / 33.1, 64x128 7.5 / 8.5; FP32: 201x777 10.7 / 14.1, 64x128 6.3 / 6.6
+// it needs at once and the march's chain of planes is gone, for 92 bytes more per node (FP32;
+// g read a second time, c written and read).  Measured on a B200, us per step of one solver with
+// nothing else on the GPU, against the march at its best tile and planes per block:
+//   FP32 3D: 256x512x256 2575 / 2946 (2730 / 2968 once the 1 kW power cap acts, after some 100
+//     steps), 128x256x128 340 / 432, 64x96x64 40 / 54
+//   FP64 3D: 128x256x128 868 / 1086, 97x131x83 305 / 396, 64x96x64 92 / 137
+//   2D, FP64: 256x1024 25.3 / 32.8, 64x128 6.0 / 8.3; FP32: 201x777 10.0 / 14.0, 64x128 5.7 / 7.0
 // Cutting a 3D grid into chunks of planes, so that the second read of g comes from L2, did not
 // pay: each chunk's two launches drain the GPU (16 planes: 2.72 ms, 64: 2.66, all: 2.66).
 //

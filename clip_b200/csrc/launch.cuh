@@ -361,14 +361,16 @@ struct Launch {
         }
     }
 
-    // Launch variant of a new solver: the two-pass step.  Measured on a B200, us per step, against
-    // the best of the marching variants at its best planes or rows per block:
-    //   3D FP32: 32x48x32 12.6 / 21.7, 64x96x64 41 / 54, 97x131x83 in walls 118 / 161, 128x256x128
-    //     339 / 429, 256x512x256 2574 / 2921, 64x160x64 with inlet and outflow 129 / 215
-    //   3D FP64: 32x48x32 20 / 29, 64x96x64 93 / 137, 97x131x83 in walls 305 / 395, 128x256x128
-    //     876 / 1083, 256^3 3508 / 4173, 64x160x64 with inlet and outflow 263 / 419
-    //   2D FP32: 64x128 6.3 / 6.6, 201x777 10.7 / 14.1, 256x1024 12.5 / 14.3, 1024x4096 159 / 169
-    //   2D FP64: 64x128 7.5 / 8.5, 201x777 18.5 / 27.1, 256x1024 26.5 / 33.1, 1024x4096 455 / 552
+    // Launch variant of a new solver: the two-pass step.  Measured on a B200, us per step of one
+    // solver with nothing else on the GPU (graphs launched once before), against the best of the
+    // marching variants at its best planes or rows per block:
+    //   3D FP32: 32x48x32 11.5 / 16.9, 64x96x64 40 / 54, 97x131x83 in walls 119 / 162, 128x256x128
+    //     340 / 432, 256x512x256 2575 / 2946 (power-capped 2730 / 2968), 64x160x64 with inlet and
+    //     outflow 127 / 215
+    //   3D FP64: 32x48x32 18.7 / 28, 64x96x64 92 / 137, 97x131x83 in walls 305 / 396, 128x256x128
+    //     868 / 1086, 256^3 3437 / 4113, 64x160x64 with inlet and outflow 260 / 431
+    //   2D FP32: 64x128 5.7 / 7.0, 201x777 10.0 / 14.0, 256x1024 11.7 / 14.1, 1024x4096 158 / 172
+    //   2D FP64: 64x128 6.0 / 8.3, 201x777 17.2 / 26.9, 256x1024 25.3 / 32.8, 1024x4096 451 / 550
     static constexpr int kTwoPass3 = PR::kExact ? 4 : 7, kTwoPass2 = 3;
     static int two_pass_variant(const DevState& st) { return st.g.dim == 3 ? kTwoPass3 : kTwoPass2; }
     static bool two_pass(const DevState& st, int variant) { return variant == two_pass_variant(st); }
@@ -448,8 +450,8 @@ struct Launch {
         monitor_final<A><<<1, 32, 0, s>>>(st.red, st.red_blocks, st.err, out2);
         return cudaGetLastError();
     }
-    // the variants whose 3D step runs step3d_body (all but the staged ones), on cases without
-    // free-convect or Neumann sides (the monitored instances carry no open-side code)
+    // the variants whose 3D step can sum the monitors as it stores (all but the staged ones), on
+    // cases without free-convect or Neumann sides (the monitored instances carry no open-side code)
     static bool fused_monitors(const DevState& st) {
         return st.g.dim == 3 && !st.g.open && st.variant != 5 && st.variant != 6 && st.variant != 9;
     }

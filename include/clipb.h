@@ -358,7 +358,8 @@ int clipb_adjoint(clipb_solver* s, const double* c0, int nsteps, const double* t
                   double* J, double* grad_c0, double* grad_params3);
 
 /* ---------------------------------------------------------------- batched 2D cases
- * Many independent 2D cases advanced together: one persistent launch per time step over
+ * Many independent 2D cases advanced together: two launches per time step (FP32/FP16), or
+ * one persistent launch, over
  * a packed table of every case's step arguments and a list of work items (case, tile,
  * row segment), replayed from a CUDA graph.  No counterpart in the reference, which runs
  * one case per process (src/main.cu:39-92); each case has exactly the semantics of a
